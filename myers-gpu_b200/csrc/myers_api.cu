@@ -295,6 +295,55 @@ static bool small_batch(uint64_t n) {
   return n > 0 && n < threshold;
 }
 
+// Whether a batch of n candidates whose lengths are flagged in present_m takes
+// bit-sliced shapes (myers_sliced.cuh) for its reads of kSlicedMinRows..
+// kSlicedMaxRows bases. A tile of theirs is 32 candidates or more on one warp
+// (on two to eight warps beyond 1,024 bases), so a batch has to fill the
+// device with such tiles. Measured, word-parallel against bit-sliced:
+//  * one length, which ends with whole rounds of tiles: 1,000 bases 33K
+//    candidates (0.87 of a round) 0.97 -> 0.85 ms, 330K 8.8 -> 6.6; 400 bases
+//    330K 1.50 -> 1.22; 100 bases 330K (1.1 rounds) 0.159 -> 0.152, 1.1M 0.446 ->
+//    0.386; 3,000 bases 11K (1.16 rounds) 3.20 -> 3.44, 44K 11.7 -> 8.5; 8,000
+//    bases 4.4K (0.93) 8.6 -> 6.0;
+//  * mixed lengths, where a round of the longest tiles comes on top: 100..1,000
+//    bases 88K 0.76 -> 0.97, 220K 1.73 -> 1.48; 1,000..10,000 bases 15K 10.9 ->
+//    11.7, 40K 25.9 -> 18.4;
+//  * the plain path's one-lane shapes of more than 16 words, and its launch per
+//    shape, need as many candidates: 1,000 bases 3.3K 0.67 -> 0.54; 35..301
+//    bases 5K 0.21 -> 0.19, 300K 0.58 -> 0.43.
+// MYERS_SLICED=0 turns the shapes off, 1 takes them for every batch.
+static int sliced_force() {
+  static const int force = [] {
+    const char* env = getenv("MYERS_SLICED");
+    return env && *env ? atoi(env) : -1;
+  }();
+  return force;
+}
+// Whether a batch of n candidates may take them at all: its lengths have to be
+// listed only then.
+static bool sliced_possible(uint64_t n) { return sliced_force() >= 0 ? sliced_force() > 0 : n >= 4096; }
+static bool sliced_batch(const uint8_t* present_m, bool batched, uint64_t n) {
+  if (!sliced_possible(n)) return false;
+  if (sliced_force() > 0) return true;
+  uint32_t lo = 0, hi = 0;
+  for (uint32_t m = kSlicedMinRows; m <= kSlicedMaxRows; ++m)
+    if (present_m[m]) {
+      if (lo == 0) lo = m;
+      hi = m;
+    }
+  if (hi == 0) return false;
+  int lg, R, lg_lo, R_lo;
+  const bool one = sliced_shape(lo, &lg_lo, &R_lo) == sliced_shape(hi, &lg, &R);
+  const uint64_t per = 32u << (lg < 5 ? 5 - lg : 0), nw = lg > 5 ? 1u << (lg - 5) : 1u;
+  const uint64_t round = 148u * (uint64_t)kSlicedWarps[sliced_class(Shape{kSlicedVariant, (uint8_t)lg, (uint8_t)R, 0})] / nw;
+  const uint64_t tiles = (n + per - 1) / per;
+  if (!one) return tiles >= 4 * round || (!batched && hi <= 1024);
+  const uint64_t rounds = (tiles + round - 1) / round;
+  if (!batched && hi > 512 && hi <= 1024 && rounds <= 1) return true;
+  if (hi <= 512 && rounds < 2) return false;
+  return rounds >= 4 || 4 * tiles >= 3 * rounds * round;
+}
+
 // lane_words > 0 asks for latency-oriented shapes: a query of more than
 // lane_words words is spread over ceil(words / W) lanes of W <= lane_words
 // words, the cheapest such shape by the cost model (shorter per-candidate
@@ -354,9 +403,10 @@ static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words = 0, bool 
 // Build the plan for the word counts flagged in `present` (size kMaxWords+1).
 // Uses fixed-size stack arrays only: no allocation on the send path.
 int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, uint64_t n,
-                      uint64_t reads) {
+                      uint64_t reads, const uint8_t* present_m, bool bucketed, uint64_t sliced_n) {
   memset(&t, 0, sizeof(t));
   memset(t.cfg_of_words, kNoCfg, sizeof(t.cfg_of_words));
+  memset(t.cfg_of_sliced, kNoCfg, sizeof(t.cfg_of_sliced));
   Shape shapes[kMaxCfg];
   uint32_t max_words[kMaxCfg];
   int16_t cfg_of[kMaxWords + 1];
@@ -368,8 +418,39 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   // of more than 16 words, and runs its lanes in two rounds. Lanes of at most
   // 16 words stage each lane's own words instead.
   const bool distinct = lane_words == 0 && reads > 0 && n < 2 * reads;
+  // Bit-sliced shapes: for the word counts without an override, every length
+  // of a word count that is present (lengths the caller did not announce but
+  // whose word count occurs are admitted, as by the word-parallel shapes).
+  const bool sliced = present_m != nullptr && lane_words == 0 && sliced_batch(present_m, batched, sliced_n ? sliced_n : n);
+  uint8_t sliced_words[kMaxWords + 1];
+  memset(sliced_words, 0, sizeof(sliced_words));
+  uint32_t sliced_rows[kSlicedShapes];  // longest length of each bit-sliced shape
+  memset(sliced_rows, 0, sizeof(sliced_rows));
+  if (sliced) {
+    std::lock_guard<std::mutex> lk(g_override_mu);
+    for (uint32_t w = kSlicedMinRows / 32 + 1; w <= kSlicedMaxRows / 32; ++w)
+      sliced_words[w] = present[w] && !g_override[batched ? 1 : 0][w].set;
+  }
+  bool alone = sliced && !bucketed;  // every length present has the same bit-sliced shape
+  int alone_shape = -1;
+  uint32_t w_lo = 0, w_hi = 0;
   for (uint32_t w = 1; w <= kMaxWords; ++w) {
     if (!present[w]) continue;
+    if (w_lo == 0) w_lo = w;
+    w_hi = w;
+    if (sliced_words[w]) {
+      t.cfg_of_words[w] = kSlicedCfg;
+      for (uint32_t m = 32 * (w - 1) + 1; m <= 32 * w; ++m) {
+        int lg, R;
+        const int i = sliced_shape(m, &lg, &R);
+        sliced_rows[i] = m;
+        if (!present_m[m]) continue;
+        if (alone_shape >= 0 && alone_shape != i) alone = false;
+        alone_shape = i;
+      }
+      continue;
+    }
+    alone = false;
     uint32_t lw = lane_words;
     if (small && w <= 32) lw = kSmallBatchLaneWords;
     else if (distinct && w > kDistinctLaneWords && w <= 32) lw = kDistinctLaneWords;
@@ -387,13 +468,45 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     if (w > max_words[found]) max_words[found] = w;
     cfg_of[w] = (int16_t)found;
   }
-  // order: persistent-kernel shapes first, each group by decreasing cost
+  alone = alone && alone_shape >= 0;
+  for (int i = 0; i < kSlicedShapes; ++i) {
+    if (sliced_rows[i] == 0 || (alone && i != alone_shape)) continue;
+    if (nshapes == kMaxCfg) return MYERS_E_QUERY_TOO_LONG;
+    int lg, R;
+    sliced_shape(sliced_rows[i], &lg, &R);
+    shapes[nshapes] = Shape{kSlicedVariant, (uint8_t)lg, (uint8_t)R, 0};
+    max_words[nshapes] = sliced_rows[i];
+    ++nshapes;
+  }
+  if (alone) {
+    // One shape for every candidate, so no bucketing: admit the lengths the
+    // word-parallel shape would (all that fit its rows on the plain path, the
+    // word counts present on the batched path).
+    t.row_min = 1;
+    t.row_limit = 32 * w_hi;
+    if (batched) {
+      t.row_min = 32 * (w_lo - 1) + 1;
+    } else {
+      const Shape s = pick_shape(w_hi, batched, distinct && w_hi > kDistinctLaneWords && w_hi <= 32 ? kDistinctLaneWords : 0,
+                                 large_batch(n));
+      t.row_limit = 32u * s.W * s.L;
+    }
+  }
+  // order: persistent-kernel shapes first, then bit-sliced ones, then the rest,
+  // each group by decreasing cost
   int order[kMaxCfg];
   double cost[kMaxCfg];
-  bool group[kMaxCfg];
+  int group[kMaxCfg];
   for (int i = 0; i < nshapes; ++i) {
     order[i] = i;
-    group[i] = !batched_supports(shapes[i].variant);
+    if (shapes[i].variant == kSlicedVariant) {
+      group[i] = 1;
+      // groups of several warps first (the kernel regroups its warps at most
+      // three times), then a tile's rows per lane times its columns
+      cost[i] = (shapes[i].L > 5 ? 1e9 * (1 << (shapes[i].L - 5)) : 0.0) + (double)shapes[i].W * max_words[i];
+      continue;
+    }
+    group[i] = batched_supports(shapes[i].variant) ? 0 : 2;
     cost[i] = shape_cost(shapes[i].variant, shapes[i].L) * max_words[i];
   }
   auto before = [&](int a, int b) { return group[a] != group[b] ? group[a] < group[b] : cost[a] > cost[b]; };
@@ -409,7 +522,12 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   for (int r = 0; r < nshapes; ++r) {
     rank[order[r]] = r;
     t.shape[r] = shapes[order[r]];
-    if (batched_supports(t.shape[r].variant)) t.num_batched = (uint32_t)r + 1;
+    if (group[order[r]] == 0) t.num_batched = (uint32_t)r + 1;
+    if (group[order[r]] == 1) {
+      ++t.num_sliced;
+      int lg, R;
+      t.cfg_of_sliced[sliced_shape(max_words[order[r]], &lg, &R)] = (uint8_t)r;
+    }
   }
   for (uint32_t w = 1; w <= kMaxWords; ++w)
     if (cfg_of[w] >= 0) t.cfg_of_words[w] = (uint8_t)rank[cfg_of[w]];
@@ -524,15 +642,23 @@ int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* presen
   uint8_t w1[kMaxWords + 1], w2[kMaxWords + 1];
   memset(w1, 0, sizeof(w1));
   memset(w2, 0, sizeof(w2));
+  std::vector<uint8_t> m1(kMaxWords * 32 + 1, 0), m2(kMaxWords * 32 + 1, 0);
   for (uint32_t m = 1; m <= kMaxWords * 32; ++m) {
     if (!present_m[m]) continue;
     const uint32_t r = host_prefix_rows(m, cutoff, mult);
+    m1[r] = 1;
     w1[(r + 31) / 32] = 1;
-    if (r < m) w2[(m + 31) / 32] = 1;
+    if (r < m) m2[m] = w2[(m + 31) / 32] = 1;
   }
-  const int st = build_plan(plan, w1, batched, 0, n);
   // the second pass holds the candidates that survived, mostly one per read
-  return st != MYERS_SUCCESS ? st : build_plan(plan2, w2, batched, 0, n, n);
+  auto both = [&](bool bucketed) {
+    const int st = build_plan(plan, w1, batched, 0, n, 0, m1.data(), bucketed);
+    return st != MYERS_SUCCESS ? st : build_plan(plan2, w2, batched, 0, n, n, m2.data(), bucketed, n / 8);
+  };
+  int st = both(batched);
+  // more than one shape in either pass: both are classified
+  if (st == MYERS_SUCCESS && !batched && (plan.num_cfg > 1 || plan2.num_cfg > 1)) st = both(true);
+  return st;
 }
 
 extern "C" uint32_t myersContextLastLaunches(const myersContext_t* c) { return c ? c->last_launches : 0; }
@@ -571,30 +697,49 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
     const Shape sh = plan.shape[c];
     return launch_plain(sh.variant, sh.L, in, ids, st, (int)c, 0, count, next, s, ctx->num_sms);
   };
-  // Plain launches of shapes c0..c1-1 of `pl` over the lists in `st`. With
-  // more than one shape they are spread over the context's streams, forked
-  // from s and joined back to it: each launch ends in a partial wave, which
-  // the other shapes' launches fill.
-  auto plain_range = [&](const PlanTable& pl, const DevInputs& din, uint32_t c0, uint32_t c1, const uint32_t* ids,
-                         BucketState* st) -> cudaError_t {
-    const uint32_t k = c1 - c0 < (uint32_t)plain_streams() ? c1 - c0 : (uint32_t)plain_streams();
+  // The launches of `pl` over the lists in `st`, but the persistent kernel's:
+  // one per class of bit-sliced shapes, then plain launches of the other shapes
+  // from c0. More than one are spread over the context's streams, forked from
+  // s and joined back to it: each ends in a partial wave, which the others
+  // fill.
+  auto shapes_enqueue = [&](const PlanTable& pl, const DevInputs& din, const uint32_t* ids, BucketState* st,
+                            uint32_t c0, uint32_t* launches) -> cudaError_t {
+    const uint32_t s0 = pl.num_batched, s1 = s0 + pl.num_sliced;
+    struct Launch { int cls; uint32_t shape; };
+    Launch list[kSlicedClasses + kMaxCfg];
+    uint32_t n = 0;
+    for (uint32_t c = s0; c < s1; ++c) {
+      const int cls = sliced_class(pl.shape[c]);
+      bool listed = false;
+      for (uint32_t i = 0; i < n; ++i) listed |= list[i].cls == cls;
+      if (!listed) list[n++] = Launch{cls, 0};
+    }
+    for (uint32_t c = c0; c < pl.num_cfg; ++c)
+      if (c < s0 || c >= s1) list[n++] = Launch{-1, c};
+    *launches += n;
+    auto one = [&](const Launch& l, cudaStream_t on) {
+      if (l.cls >= 0) return launch_sliced(l.cls, din, ids, pl, st, s0, s1, 0, nullptr, on, ctx->num_sms);
+      return launch_plain(pl.shape[l.shape].variant, pl.shape[l.shape].L, din, ids, st, (int)l.shape, 0, 0,
+                          &st->next[l.shape], on, ctx->num_sms);
+    };
+    const uint32_t k = n < (uint32_t)plain_streams() ? n : (uint32_t)plain_streams();
     cudaError_t e = cudaSuccess;
     if (k <= 1 || ctx->aux[0] == nullptr) {
-      for (uint32_t c = c0; c < c1 && e == cudaSuccess; ++c)
-        e = launch_plain(pl.shape[c].variant, pl.shape[c].L, din, ids, st, (int)c, 0, 0, &st->next[c], s,
-                         ctx->num_sms);
+      for (uint32_t i = 0; i < n && e == cudaSuccess; ++i) e = one(list[i], s);
       return e;
     }
     e = cudaEventRecord(ctx->fork, s);
     for (uint32_t i = 0; i < k && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(ctx->aux[i], ctx->fork, 0);
-    for (uint32_t c = c0; c < c1 && e == cudaSuccess; ++c)
-      e = launch_plain(pl.shape[c].variant, pl.shape[c].L, din, ids, st, (int)c, 0, 0, &st->next[c],
-                       ctx->aux[(c - c0) % k], ctx->num_sms);
+    for (uint32_t i = 0; i < n && e == cudaSuccess; ++i) e = one(list[i], ctx->aux[i % k]);
     for (uint32_t i = 0; i < k && e == cudaSuccess; ++i) {
       e = cudaEventRecord(ctx->join[i], ctx->aux[i]);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ctx->join[i], 0);
     }
     return e;
+  };
+  // The launch of a plan that is one bit-sliced shape, over every candidate.
+  auto sliced_launch = [&](const PlanTable& pl, const DevInputs& din, uint32_t* next) {
+    return launch_sliced(sliced_class(pl.shape[0]), din, nullptr, pl, nullptr, 0, 1, din.num_cands, next, s, ctx->num_sms);
   };
   if (in.cut && path == MYERS_PATH_BATCHED && plan2 != nullptr) {
     // The cut-off's two passes as two persistent launches: the first over
@@ -616,10 +761,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
       CU(launch_batched(in, ctx->d_ids, plan, ctx->d_state, s, ctx->num_sms, batched_tile_bound(plan, in.num_cands)));
       ++launches;
     }
-    for (uint32_t c = plan.num_batched; c < plan.num_cfg; ++c) {
-      CU(plain(c, ctx->d_ids, ctx->d_state, 0, &ctx->d_state->next[c]));
-      ++launches;
-    }
+    CU(shapes_enqueue(plan, in, ctx->d_ids, ctx->d_state, plan.num_batched, &launches));
     DevInputs in2 = in;
     in2.prefix = 0;
     CU(launch_plan_tiles(*plan2, ctx->d_esc_state, s));
@@ -629,12 +771,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
                         batched_tile_bound(*plan2, in.num_cands)));
       ++launches;
     }
-    for (uint32_t c = plan2->num_batched; c < plan2->num_cfg; ++c) {
-      const Shape sh = plan2->shape[c];
-      CU(launch_plain(sh.variant, sh.L, in2, ctx->d_esc_ids, ctx->d_esc_state, (int)c, 0, 0,
-                      &ctx->d_esc_state->next[c], s, ctx->num_sms));
-      ++launches;
-    }
+    CU(shapes_enqueue(*plan2, in2, ctx->d_esc_ids, ctx->d_esc_state, plan2->num_batched, &launches));
     ctx->last_launches = launches;
     return MYERS_SUCCESS;
   }
@@ -655,7 +792,8 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
       if (plan.num_cfg == 1) {
         uint32_t* next = &ctx->d_state->next[0];
         CU(cudaMemsetAsync(next, 0, sizeof(uint32_t), s));
-        CU(plain(0, nullptr, nullptr, in.num_cands, next));
+        if (plan.num_sliced == 1) CU(sliced_launch(plan, in, next));
+        else CU(plain(0, nullptr, nullptr, in.num_cands, next));
         ++launches;
       }
     } else {
@@ -665,17 +803,22 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
       launches += (uint32_t)launch_bucketing_cutoff(in, plan, *plan2, ctx->d_state, ctx->d_cfg, ctx->d_ids, s,
                                                     ctx->num_sms, &e);
       if (e != cudaSuccess) return cuda_fail(e, "bucketing");
-      CU(plain_range(plan, in, 0, plan.num_cfg, ctx->d_ids, ctx->d_state));
-      launches += plan.num_cfg;
+      CU(shapes_enqueue(plan, in, ctx->d_ids, ctx->d_state, 0, &launches));
     }
     DevInputs in2 = in;
     in2.prefix = 0;
-    CU(plain_range(*plan2, in2, 0, plan2->num_cfg, ctx->d_esc_ids, ctx->d_esc_state));
-    launches += plan2->num_cfg;
+    CU(shapes_enqueue(*plan2, in2, ctx->d_esc_ids, ctx->d_esc_state, 0, &launches));
     ctx->last_launches = launches;
     return MYERS_SUCCESS;
   }
-  if (path == MYERS_PATH_PLAIN && plan.num_cfg == 1) {
+  if (sliced_alone(plan)) {
+    uint32_t* next = &ctx->d_state->next[0];  // the launch's tile counter
+    CU(cudaMemsetAsync(next, 0, sizeof(uint32_t), s));
+    CU(sliced_launch(plan, in, next));
+    ctx->last_launches = 1;
+    return MYERS_SUCCESS;
+  }
+  if (path == MYERS_PATH_PLAIN && plan.num_cfg == 1 && plan.num_sliced == 0) {
     uint32_t* next = &ctx->d_state->next[0];  // the launch's tile counter
     CU(cudaMemsetAsync(next, 0, sizeof(uint32_t), s));
     CU(plain(0, nullptr, nullptr, in.num_cands, next));
@@ -692,8 +835,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
     ++launches;
     first_plain = plan.num_batched;
   }
-  CU(plain_range(plan, in, first_plain, plan.num_cfg, ctx->d_ids, ctx->d_state));
-  launches += plan.num_cfg - first_plain;
+  CU(shapes_enqueue(plan, in, ctx->d_ids, ctx->d_state, first_plain, &launches));
   ctx->last_launches = launches;
   return MYERS_SUCCESS;
 }
@@ -706,7 +848,10 @@ static int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, i
   if (maxSize > kMaxWords * 32) maxSize = kMaxWords * 32;
   const uint32_t wlo = minSize ? (minSize + 31) / 32 : 1, whi = (maxSize + 31) / 32;
   for (uint32_t w = wlo; w <= whi; ++w) present[w] = 1;
-  return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, n, reads);
+  if (!sliced_possible(n)) return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, n, reads);
+  std::vector<uint8_t> present_m(kMaxWords * 32 + 1, 0);
+  for (uint32_t m = minSize ? minSize : 1; m <= maxSize; ++m) present_m[m] = 1;
+  return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, n, reads, present_m.data());
 }
 
 extern "C" int myersVerifyAsync(myersContext_t* ctx, const myersReference_t* ref, const qryEntry_t* d_peq,
@@ -959,7 +1104,7 @@ struct Buffer {
   int last_status;
   bool pending;
   std::vector<uint8_t> present;    // word counts of the last send
-  std::vector<uint8_t> present_m;  // query lengths of the last send (cut-off only)
+  std::vector<uint8_t> present_m;  // query lengths of the last send
   PlanTable plan, plan2;
   bool plan_valid;
   int plan_path;
@@ -1071,6 +1216,7 @@ extern "C" int myersInit(void*** myersBuffer, uint32_t numBuffers, const char* r
     const char* g = getenv("MYERS_GRAPHS");
     b->use_graphs = !(g && strcmp(g, "0") == 0);
     b->present.assign(kMaxWords + 1, 0);
+    b->present_m.assign(kMaxWords * 32 + 1, 0);
     bufs[i] = b;
     st = buffer_alloc(b);
     if (st != MYERS_SUCCESS) {
@@ -1101,27 +1247,27 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
   CU(cudaSetDevice(b->device));
   // O(queries) host pass: the word counts present pick the shapes
   std::vector<uint8_t>& present = b->present;
+  std::vector<uint8_t>& pm = b->present_m;
+  const bool two_pass = b->cutoff >= 0.0f;
+  const bool lengths = two_pass || sliced_possible(numCandidates);  // ... and the lengths, where they can matter
   std::fill(present.begin(), present.end(), 0);
+  if (lengths) std::fill(pm.begin(), pm.end(), 0);
   for (uint32_t q = 0; q < numQueries; ++q) {
     const uint32_t m = b->h_qinfo[q].size;
-    if (m > 0 && m <= kMaxWords * 32) present[(m + 31) / 32] = 1;  // longer: flagged on the device
+    if (m == 0 || m > kMaxWords * 32) continue;  // longer: flagged on the device
+    present[(m + 31) / 32] = 1;
+    if (lengths) pm[m] = 1;
   }
   PlanTable& plan = b->plan;
-  const bool two_pass = b->cutoff >= 0.0f;
   int st;
   {
     NvtxRange plan_range("myers: send: shape plan");
     if (two_pass) {
-      std::vector<uint8_t>& pm = b->present_m;
-      pm.assign(kMaxWords * 32 + 1, 0);
-      for (uint32_t q = 0; q < numQueries; ++q) {
-        const uint32_t m = b->h_qinfo[q].size;
-        if (m > 0 && m <= kMaxWords * 32) pm[m] = 1;
-      }
       st = cutoff_plans(plan, b->plan2, pm.data(), b->cutoff, cutoff_prefix_mult(), b->path == MYERS_PATH_BATCHED,
                         numCandidates);
     } else {
-      st = build_plan(plan, present.data(), b->path == MYERS_PATH_BATCHED, 0, numCandidates, numQueries);
+      st = build_plan(plan, present.data(), b->path == MYERS_PATH_BATCHED, 0, numCandidates, numQueries,
+                      lengths ? pm.data() : nullptr);
     }
   }
   if (st != MYERS_SUCCESS) return b->last_status = st;
@@ -1178,7 +1324,8 @@ extern "C" int myersReceive(void* mb) {
   CU(cudaStreamSynchronize(b->stream));
   if (b->pending) {
     b->pending = false;
-    if (*b->h_flags != 0) b->last_status = MYERS_E_QUERY_TOO_LONG;
+    if (*b->h_flags & kFlagTimeout) b->last_status = MYERS_E_TIMEOUT;
+    else if (*b->h_flags != 0) b->last_status = MYERS_E_QUERY_TOO_LONG;
   }
   return b->last_status;
 }
@@ -1373,11 +1520,24 @@ extern "C" int myersVerifyNoAllocAsync(const uint32_t* d_refWords, uint64_t refW
   CU(cudaMemsetAsync(d_state, 0, sizeof(BucketState), s));
   CU(cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), s));
   cudaError_t e = cudaSuccess;
+  if (sliced_alone(plan)) {
+    CU(launch_sliced(sliced_class(plan.shape[0]), in, nullptr, plan, nullptr, 0, 1, numCandidates, &d_state->next[0], s,
+                     dev.num_sms));
+    return MYERS_SUCCESS;
+  }
   launch_bucketing(in, plan, d_state, d_cfg, d_ids, s, dev.num_sms, &e);
   if (e != cudaSuccess) return cuda_fail(e, "bucketing");
   if (plan.num_batched > 0)
     CU(launch_batched(in, d_ids, plan, d_state, s, dev.num_sms, batched_tile_bound(plan, numCandidates)));
-  for (uint32_t c = plan.num_batched; c < plan.num_cfg; ++c)
+  for (int cls = 0; cls < kSlicedClasses; ++cls) {
+    bool any = false;
+    for (uint32_t c = plan.num_batched; c < plan.num_batched + plan.num_sliced; ++c)
+      any |= sliced_class(plan.shape[c]) == cls;
+    if (any)
+      CU(launch_sliced(cls, in, d_ids, plan, d_state, plan.num_batched, plan.num_batched + plan.num_sliced, 0, nullptr, s,
+                       dev.num_sms));
+  }
+  for (uint32_t c = plan.num_batched + plan.num_sliced; c < plan.num_cfg; ++c)
     CU(launch_plain(plan.shape[c].variant, plan.shape[c].L, in, d_ids, d_state, (int)c, 0, 0, &d_state->next[c], s,
                     dev.num_sms));
   return MYERS_SUCCESS;

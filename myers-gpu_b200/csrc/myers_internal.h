@@ -32,6 +32,7 @@ constexpr uint32_t kMaxColumns = 65535;       // the result key keeps 16 column 
 constexpr uint32_t kFlagUnsupported = 1u;     // query too long or window too wide
 constexpr uint32_t kFlagBadQuery = 2u;        // candidate query index >= numQueries
 constexpr uint32_t kFlagBadEntry = 4u;        // query PEQ entries beyond numPEQEntries
+constexpr uint32_t kFlagTimeout = 8u;         // a bounded wait inside a kernel gave up
 
 // Candidate as laid out by the API (candInfo_t with its 4 padding bytes).
 struct Cand {
@@ -66,7 +67,7 @@ struct Shape {
   uint8_t pad;
 };
 
-constexpr int kMaxCfg = 128;            // distinct shapes in one plan
+constexpr int kMaxCfg = 240;            // distinct shapes in one plan
 // Batches of at least this many candidates take the batched path's shapes for
 // large batches (every lane width; the autotuner cache's "batched_large").
 constexpr uint64_t kLargeBatchCandidates = 150000;
@@ -81,17 +82,50 @@ constexpr uint32_t kDistinctLaneWords = 16;
 constexpr int kPlainStreams = 4;
 constexpr uint8_t kNoCfg = 0xFF;
 
+// Bit-sliced shapes (myers_sliced.cuh): Shape{kSlicedVariant, log2 of the lanes
+// per group of 32 candidates, rows per lane}. The lanes are the smallest of
+// 8, 16, .. 256 that need at most 32 rows each (40 with 256 lanes, in steps of
+// two above 32).
+constexpr uint8_t kSlicedVariant = 0xFE;
+constexpr uint8_t kSlicedCfg = 0xFE;    // cfg_of_words: look in cfg_of_sliced
+constexpr uint32_t kSlicedMinRows = 65, kSlicedMaxRows = 10240;
+constexpr int kSlicedMinLg = 3, kSlicedMaxLg = 8, kSlicedMinR = 9, kSlicedMaxR = 40;
+constexpr int kSlicedShapes = (kSlicedMaxLg - kSlicedMinLg + 1) * (kSlicedMaxR - kSlicedMinR + 1);
+
+// Index of the bit-sliced shape of m rows (kSlicedMinRows..kSlicedMaxRows).
+__host__ __device__ inline int sliced_shape(uint32_t m, int* lg, int* R) {
+  int g = kSlicedMinLg;
+  while (g < kSlicedMaxLg && m > (32u << g)) ++g;
+  int r = (int)((m + (1u << g) - 1u) >> g);
+  if (r > 32) r += r & 1;
+  *lg = g;
+  *R = r;
+  return (g - kSlicedMinLg) * (kSlicedMaxR - kSlicedMinR + 1) + r - kSlicedMinR;
+}
+
 // Per-send plan, passed by value as a __grid_constant__ kernel parameter:
 // word count -> shape index, and the shapes in launch order. The first
 // num_batched shapes (most expensive first) go to the persistent kernel on
-// the batched path; the rest always get plain launches.
+// the batched path, the next num_sliced to the bit-sliced kernel on both
+// paths; the rest always get plain launches.
 struct PlanTable {
   uint8_t cfg_of_words[kMaxWords + 1];
-  uint8_t pad[3];
+  uint8_t cfg_of_sliced[kSlicedShapes];
   uint32_t num_cfg;
   uint32_t num_batched;
+  uint32_t num_sliced;
+  uint32_t row_min, row_limit;  // one bit-sliced shape without bucketing: the queries it admits (else 0, 0)
   Shape shape[kMaxCfg];
 };
+
+// The shape of m rows (1..kMaxWords * 32) under a plan, or kNoCfg.
+__host__ __device__ inline uint32_t plan_cfg(const PlanTable& plan, uint32_t m) {
+  const uint32_t c = plan.cfg_of_words[(m + 31) >> 5];
+  if (c != kSlicedCfg) return c;
+  if (m < kSlicedMinRows || m > kSlicedMaxRows) return kNoCfg;
+  int lg, R;
+  return plan.cfg_of_sliced[sliced_shape(m, &lg, &R)];
+}
 
 // Device-computed layout of the bucketed candidate list.
 struct BucketState {
@@ -153,7 +187,9 @@ inline void set_multipliers(DevInputs& in) {
 
 inline int variant_W(int v) { return v < kNumSingle ? v + 1 : kMultiW[v - kNumSingle]; }
 inline bool variant_multi(int v) { return v >= kNumSingle; }
-inline bool batched_supports(int v) { return !variant_multi(v) || variant_W(v) <= kBatchedMaxMultiW; }
+inline bool batched_supports(int v) {
+  return v != kSlicedVariant && (!variant_multi(v) || variant_W(v) <= kBatchedMaxMultiW);
+}
 
 // ---- host launchers (myers_kernels.cu) ----
 
@@ -188,6 +224,40 @@ cudaError_t launch_plan_tiles(const PlanTable& plan2, BucketState* d_esc_state, 
 cudaError_t launch_batched(const DevInputs& in, const uint32_t* d_ids, const PlanTable& plan,
                            BucketState* d_state, cudaStream_t s, int num_sms, uint32_t max_tiles);
 
+// The bit-sliced kernels (myers_sliced.cuh), one per class of shapes.
+constexpr int kSlicedClasses = 4;
+inline int sliced_class(const Shape& s) { return s.L > 5 ? 3 : s.W <= 16 ? 0 : s.W <= 24 ? 1 : 2; }
+constexpr int kSlicedWarps[kSlicedClasses] = {16, 12, 8, 8};  // warps per SM
+// A launch over the class's shapes among shapes c0..c1-1 of the plan, their lists
+// in d_state (whose next counters start at zero); with d_state == nullptr over
+// candidates 0..count-1 as shape c0, with the tile counter d_next (zero when
+// the launch starts).
+template <int CLASS>
+cudaError_t launch_sliced_class(const DevInputs& in, const uint32_t* d_ids, const PlanTable& plan, BucketState* d_state,
+                                uint32_t c0, uint32_t c1, uint32_t count, uint32_t* d_next, cudaStream_t s, int num_sms);
+template <int CLASS>
+const void* sliced_class_kernel();
+template <> cudaError_t launch_sliced_class<0>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> cudaError_t launch_sliced_class<1>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> cudaError_t launch_sliced_class<2>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> cudaError_t launch_sliced_class<3>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> const void* sliced_class_kernel<0>();
+template <> const void* sliced_class_kernel<1>();
+template <> const void* sliced_class_kernel<2>();
+template <> const void* sliced_class_kernel<3>();
+inline cudaError_t launch_sliced(int cls, const DevInputs& in, const uint32_t* d_ids, const PlanTable& plan,
+                                 BucketState* d_state, uint32_t c0, uint32_t c1, uint32_t count, uint32_t* d_next,
+                                 cudaStream_t s, int num_sms) {
+  switch (cls) {
+    case 0: return launch_sliced_class<0>(in, d_ids, plan, d_state, c0, c1, count, d_next, s, num_sms);
+    case 1: return launch_sliced_class<1>(in, d_ids, plan, d_state, c0, c1, count, d_next, s, num_sms);
+    case 2: return launch_sliced_class<2>(in, d_ids, plan, d_state, c0, c1, count, d_next, s, num_sms);
+    default: return launch_sliced_class<3>(in, d_ids, plan, d_state, c0, c1, count, d_next, s, num_sms);
+  }
+}
+// Whether the plan is one bit-sliced shape for every candidate.
+inline bool sliced_alone(const PlanTable& plan) { return plan.num_cfg == 1 && plan.num_sliced == 1 && plan.row_limit > 0; }
+
 // Load every kernel the batched path can launch (bucketing, the persistent
 // kernel, the plain launches of shapes it does not carry) on the current
 // device. With lazy module loading a kernel is otherwise loaded, and its code
@@ -213,8 +283,13 @@ cudaError_t launch_lop3_probe(uint32_t* d_out, int blocks, int threads, int iter
 // n: the batch's candidates, which picks the batched path's table for large
 // batches at kLargeBatchCandidates or more.
 // reads: how many reads the n candidates come from (0: unknown).
+// present_m: flags each query length 1..kMaxWords * 32 that can occur; with
+// it, large batches take bit-sliced shapes.
+// bucketed: the candidates will be classified by the plan in any case, so it
+// names every shape of the word counts present.
+// sliced_n: candidates expected, where they are not n (the cut-off's second pass).
 int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words = 0, uint64_t n = 0,
-               uint64_t reads = 0);
+               uint64_t reads = 0, const uint8_t* present_m = nullptr, bool bucketed = false, uint64_t sliced_n = 0);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.
 uint32_t batched_tile_bound(const PlanTable& plan, uint32_t n);
 // Record a CUDA failure (message for myersGetErrorString) and return MYERS_E_CUDA.
