@@ -426,31 +426,125 @@ __device__ __forceinline__ uint32_t ascii_code(uint32_t b) {
   return u == 'A' ? 0u : u == 'C' ? 1u : u == 'G' ? 2u : u == 'T' ? 3u : 4u;
 }
 
-// One thread per 32-base word of a read: the five 32-bit bitmaps of that
-// word. Bits past the read's end are 0 (src-api/genCandidate-reorder.c:258-317).
+// Four bases at a time. In ASCII, bits 1 and 2 tell the letters apart (A 00, C
+// 01, T 10, G 11); the byte is that letter, of either case, iff bits 7, 6 and 3
+// are 010, bit 4 is set for T alone and bit 0 for the other three alone.
+// Non-zero bits of the result: bytes that are none of the four.
+__device__ __forceinline__ uint32_t not_acgt(uint32_t w) {
+  const uint32_t t = w & 0x04040404u & ~(w * 2u);  // T: bit 2 without bit 1
+  const uint32_t x = w ^ (t * 4u + (t >> 2)) ^ 0x41414141u;
+  return x & 0xD9D9D9D9u;
+}
+// Bits 0, 8, 16 and 24 of x, times 2^p, as bits 28 .. 31.
+template <int P>
+__device__ __forceinline__ uint32_t gather4(uint32_t x) {
+  return x * (0x10204080u >> P);
+}
+
+// One lane per 32-base word, over the words of `per` consecutive reads at a
+// time: the five 32-bit bitmaps of that word. Bits past the read's end are 0
+// (src-api/genCandidate-reorder.c:258-317).
+//
+// Bound by the ALU pipe and by memory (one byte in, 0.625 out per base): the
+// bytes' two letter bits are gathered four at a time by a multiplication, and
+// the planes follow from the two gathered words; bytes that are no letter of
+// the four take a second look. 100K reads of 1,000 bases (164 MB, 25 us of
+// copying) took 176 us with a byte load and a table update per base, and take
+// 43; 1M of 100 bases 1,470 (a warp per read) and 47.
 __global__ void k_pack_peq(const uint8_t* __restrict__ ascii, unsigned long long ascii_bytes,
                            const unsigned long long* __restrict__ offsets, const uint2* __restrict__ qinfo,
                            uint32_t num_reads, uint32_t* __restrict__ peq, uint32_t num_entries,
-                           uint32_t* __restrict__ flags) {
-  const uint32_t stride = gridDim.x * (blockDim.x / 32);
+                           uint32_t* __restrict__ flags, uint32_t per) {
+  const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
   const int lane = threadIdx.x & 31;
-  for (uint32_t r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); r < num_reads; r += stride) {
-    const uint2 q = qinfo[r];
-    const unsigned long long o = offsets[r];
-    const uint32_t m = q.y;
-    const uint32_t nwords = ((m + 127) / 128) * 4;  // whole entries, padding words zeroed
-    const unsigned long long o1 = offsets[r + 1];
-    if ((unsigned long long)q.x + nwords / 4 > num_entries || o1 < o || o1 - o < m || o1 > ascii_bytes) {
-      if (lane == 0) atomicOr(flags, kFlagBadEntry);
-      continue;
+  const uint32_t batches = (num_reads + per - 1) / per;
+  for (uint32_t batch = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); batch < batches; batch += nwarps) {
+    // lane r holds read r of the batch: its words (whole entries) before and
+    // after those of the reads up to it
+    const uint32_t r = batch * per + (uint32_t)lane;
+    uint2 q = make_uint2(0u, 0u);
+    unsigned long long o = 0;
+    uint32_t words = 0;
+    if ((uint32_t)lane < per && r < num_reads) {
+      q = qinfo[r];
+      o = offsets[r];
+      const unsigned long long o1 = offsets[r + 1];
+      words = (q.y + 127) / 128 * 4;
+      if ((unsigned long long)q.x + words / 4 > num_entries || o1 < o || o1 - o < q.y || o1 > ascii_bytes) {
+        atomicOr(flags, kFlagBadEntry);
+        words = 0;
+      }
     }
-    for (uint32_t w = lane; w < nwords; w += 32) {
-      uint32_t bm[5] = {0u, 0u, 0u, 0u, 0u};
-      const uint32_t b0 = w * 32;
-      for (uint32_t i = 0; i < 32 && b0 + i < m; ++i) bm[ascii_code(ascii[o + b0 + i])] |= 1u << i;
-      uint32_t* e = peq + (size_t)(q.x + w / 4) * 20;
+    uint32_t end = words;
 #pragma unroll
-      for (int c = 0; c < 5; ++c) e[c * 4 + (w & 3)] = bm[c];
+    for (int s = 1; s < 32; s <<= 1) {
+      const uint32_t x = __shfl_up_sync(FULL_MASK, end, s);
+      if (lane >= s) end += x;
+    }
+    const uint32_t total = __shfl_sync(FULL_MASK, end, 31);
+    for (uint32_t i0 = 0; i0 < total; i0 += 32) {
+      const uint32_t i = i0 + (uint32_t)lane;
+      // the first read whose words end after i
+      int at = 0;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) {
+        const uint32_t e = __shfl_sync(FULL_MASK, end, at + s - 1);
+        if (e <= i) at += s;
+      }
+      at = min(at, 31);
+      const uint32_t m = __shfl_sync(FULL_MASK, q.y, at), entry = __shfl_sync(FULL_MASK, q.x, at);
+      const unsigned long long base = __shfl_sync(FULL_MASK, o, at);
+      const uint32_t first = __shfl_sync(FULL_MASK, end - words, at);
+      if (i >= total) continue;
+      const uint32_t w = i - first;
+      const uint32_t left = m > 32 * w ? m - 32 * w : 0u;
+      uint32_t bm[5] = {0u, 0u, 0u, 0u, 0u};
+      if (left > 0) {
+        const uint8_t* p = ascii + base + 32ull * w;
+        const uint32_t sh = 8u * (uint32_t)((uintptr_t)p & 3u);
+        const uint8_t* a = p - (sh >> 3);
+        uint32_t v[9];
+        if (a >= ascii && a + 36 <= ascii + ascii_bytes) {
+          const uint32_t* x = reinterpret_cast<const uint32_t*>(a);
+#pragma unroll
+          for (int k = 0; k < 9; ++k) v[k] = __ldg(x + k);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) v[k] = __funnelshift_r(v[k], v[k + 1], sh);
+        } else {  // at an edge of the buffer: the read's bytes alone
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            v[k] = 0u;
+            for (uint32_t b = 0; b < 4; ++b)
+              if (4u * k + b < left) v[k] |= (uint32_t)p[4 * k + b] << (8 * b);
+          }
+        }
+        uint32_t b1 = 0u, b2 = 0u, odd = 0u;
+#pragma unroll
+        for (int k = 7; k >= 0; --k) {  // in from below
+          b1 = __funnelshift_l(gather4<1>(v[k] & 0x02020202u), b1, 4);
+          b2 = __funnelshift_l(gather4<2>(v[k] & 0x04040404u), b2, 4);
+          odd |= not_acgt(v[k]);
+        }
+        const uint32_t inside = left >= 32u ? FULL_MASK : (1u << left) - 1u;
+        uint32_t n = 0u;
+        if (odd) {
+#pragma unroll
+          for (int k = 7; k >= 0; --k) {
+            const uint32_t z = not_acgt(v[k]);
+            const uint32_t other = ((((z & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | z) >> 7) & 0x01010101u;  // byte not zero
+            n = __funnelshift_l(gather4<0>(other), n, 4);
+          }
+        }
+        const uint32_t letter = inside & ~n;
+        bm[0] = letter & ~b1 & ~b2;
+        bm[1] = letter & b1 & ~b2;
+        bm[2] = letter & b1 & b2;
+        bm[3] = letter & ~b1 & b2;
+        bm[4] = inside & n;
+      }
+      uint32_t* e = peq + (size_t)(entry + w / 4) * 20 + (w & 3);
+#pragma unroll
+      for (int c = 0; c < 5; ++c) e[c * 4] = bm[c];
     }
   }
 }
@@ -475,9 +569,12 @@ cudaError_t launch_pack_peq(const uint8_t* ascii, unsigned long long ascii_bytes
                             const uint2* qinfo, uint32_t num_reads, uint32_t* peq, uint32_t num_entries,
                             uint32_t* flags, cudaStream_t s, int num_sms) {
   if (num_reads == 0) return cudaSuccess;
-  uint32_t grid = (num_reads + 7) / 8;
-  if (grid > (uint32_t)num_sms * 16) grid = (uint32_t)num_sms * 16;
-  k_pack_peq<<<grid, 256, 0, s>>>(ascii, ascii_bytes, offsets, qinfo, num_reads, peq, num_entries, flags);
+  // as many reads per warp as leave the device a few rounds of warps
+  uint32_t per = 32;
+  while (per > 1 && num_reads / per < (uint32_t)num_sms * 192) per /= 2;
+  const uint32_t warps = (num_reads + per - 1) / per;
+  const uint32_t grid = (warps + 7) / 8;
+  k_pack_peq<<<grid, 256, 0, s>>>(ascii, ascii_bytes, offsets, qinfo, num_reads, peq, num_entries, flags, per);
   return cudaGetLastError();
 }
 
