@@ -69,6 +69,8 @@ struct TbState {
   unsigned int max_units;  // largest band store (256-byte units), for any words per lane
   unsigned int max_inv_words;  // ~(shortest query's words): zero-initialised like the rest
   unsigned int next[2][2];  // per scratch half: work counters of the forward pass and the walk
+  unsigned int max_band;    // widest diagonal band (words, tb_window) of a traced candidate
+  unsigned int max_columns; // most columns of one
 };
 
 struct TbArgs {
@@ -167,13 +169,20 @@ __device__ __forceinline__ unsigned long long tb_slot_bound(const TbGeom& g) {
   return (unsigned long long)(g.c1 - g.a0 + 1u) * B * 16ull;
 }
 
+// Words of the diagonal band of a candidate of score s and `words` query words
+// in the banded kernel (see k_tb_band).
+__device__ __forceinline__ uint32_t tb_window(uint32_t s, uint32_t words) {
+  const uint32_t w = 2u * ((s + 31u) >> 5) + 1u;
+  return w < words ? w : words;
+}
+
 // Pick the candidates to trace; write the records of the others.
 __global__ void k_tb_select(TbArgs a, uint32_t* ids, unsigned long long* offs) {
   const uint32_t lane = threadIdx.x & 31u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < a.num_cands; base += gridDim.x * blockDim.x) {
     const uint32_t id = base + threadIdx.x;
     bool traced = false;
-    uint32_t units = 0;
+    uint32_t units = 0, words = 0, window = 0, columns = 0;
     TbGeom g;
     if (id < a.num_cands) {
       const uint2 res = a.results[id];
@@ -184,14 +193,26 @@ __global__ void k_tb_select(TbArgs a, uint32_t* ids, unsigned long long* offs) {
         traced = true;
         rec.y = 0u;
         units = (uint32_t)((tb_slot_bound(g) + (1ull << kTbUnitShift) - 1ull) >> kTbUnitShift);
-        atomicMax(&a.st->max_words, (g.m + 31u) >> 5);
-        atomicMax(&a.st->max_inv_words, ~((g.m + 31u) >> 5));
-        atomicMax(&a.st->max_units, units);
+        words = (g.m + 31u) >> 5;
+        window = tb_window(g.s, words);
+        columns = g.c1 - g.a0;
       }
       a.alns[id] = rec;
     }
     // warp-aggregated append: list places and band offsets in one atomic
     const uint32_t mask = __ballot_sync(FULL_MASK, traced);
+    if (mask) {  // the extremes, one atomic each per warp
+      const uint32_t w = __reduce_max_sync(FULL_MASK, words), iw = __reduce_max_sync(FULL_MASK, traced ? ~words : 0u);
+      const uint32_t u = __reduce_max_sync(FULL_MASK, units), b = __reduce_max_sync(FULL_MASK, window);
+      const uint32_t c = __reduce_max_sync(FULL_MASK, columns);
+      if (lane == 0) {
+        atomicMax(&a.st->max_words, w);
+        atomicMax(&a.st->max_inv_words, iw);
+        atomicMax(&a.st->max_units, u);
+        atomicMax(&a.st->max_band, b);
+        atomicMax(&a.st->max_columns, c);
+      }
+    }
     unsigned long long incl = units;  // inclusive prefix of the units over the warp
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -530,6 +551,318 @@ __global__ void __launch_bounds__(128) k_tb_walk(TbArgs a) {
   }
 }
 
+// ---- the banded kernel: recomputation and walk in one pass ----
+//
+// Every cell that an alignment of cost s ending in (m, c1) can use has j - i
+// within s of c1 - m, so only that band is recomputed: bits of a window of W =
+// 2 ceil(s / 32) + 1 words, which moves up one word per 32 columns counted
+// from the end column. Cells outside the window get upper bounds (the row
+// below it grows by one per column, a word that enters on top starts at +1 per
+// row, the first column at D = i). The banded matrix is then at least the true
+// one everywhere and equal to it on every optimal path, so each step of the
+// walk is decided as by the full matrix, and the end cell equals s exactly when
+// the full matrix's does.
+//
+// The walk needs two bits per cell: Dg, the diagonal step is consistent (the
+// bases match, or D(i,j) = D(i-1,j-1) + 1), and E, the match bit where it is
+// and the +1 bit of the vertical delta where it is not ('I' rather than 'D').
+//
+// One lane per candidate. A warp keeps its window's PEQ words in shared memory
+// (a word per lane and bank), runs the columns forward and saves the state
+// before every 8 columns; then it goes back block by block, recomputes 8
+// columns with the two bits in shared memory and walks through them. Nothing
+// but the saved states (W x 8 bytes per 8 columns) goes through memory, in a
+// slot per resident warp, so one launch traces everything that is traced.
+//
+// Bound by the ALU pipe. Storing the bands of a full recomputation and walking
+// them in a second kernel, a 30K-candidate call of 1,000-base reads took 3.1
+// ms; TB_FIGURES
+template <int W>
+struct BandMem {
+  static constexpr uint32_t kPeq = 6u * W * 32u;       // [base, and one that matches nothing][word][lane]
+  static constexpr uint32_t kBits = 8u * W * 32u * 2u; // [column][word][lane] {Dg, E}
+  static constexpr uint32_t kWords = kPeq + kBits;
+};
+
+struct BandLane {
+  TbGeom g;
+  uint32_t tw;      // query words
+  uint32_t nc;      // columns a0 + 1 .. c1
+  long long base;   // base index of column c1, plus one
+};
+
+// The window's first word in block b of 32 columns counted from the end.
+template <int W>
+__device__ __forceinline__ int band_first(const BandLane& c, int b) {
+  const int x = (int)c.tw - 1 - b - (W - 1) / 2;
+  return x > 0 && c.tw > (uint32_t)W ? x : 0;  // a window that holds the whole query stays
+}
+
+// Word x of the top-aligned query into place k of the window, all five bases.
+template <int W>
+__device__ __forceinline__ void band_load(const TbArgs& a, const BandLane& c, uint32_t* __restrict__ peq, int k, int x,
+                                          bool on) {
+  const uint32_t p = 32u * c.tw - c.g.m;  // < 32: padding rows that match nothing
+#pragma unroll
+  for (int b = 0; b < 5; ++b) {
+    uint32_t v = 0u;
+    if (on) {
+      const uint32_t hi = qword(a.peq, c.g.pos_entry, (int)c.tw, b, x), lo = qword(a.peq, c.g.pos_entry, (int)c.tw, b, x - 1);
+      v = p ? __funnelshift_r(lo, hi, 32 - p) : hi;
+    }
+    peq[(b * W + k) * 32] = v;
+  }
+}
+
+// The text codes of the 8 columns 8 q .. 8 q + 7 from the end, the last of them
+// first (lowest nibble), 5 for columns before the candidate's first.
+__device__ __forceinline__ uint32_t band_text(const TbArgs& a, const BandLane& c, int q) {
+  const long long b = c.base - 8ll * (q + 1);
+  const uint32_t lo = ref_load(a.ref, b >> 3, a.ref_words), hi = ref_load(a.ref, (b >> 3) + 1, a.ref_words);
+  const uint32_t t = sanitize_codes(__funnelshift_r(lo, hi, 4u * (uint32_t)(b & 7)));
+  const int before = 8 * q + 8 - (int)c.nc;
+  const uint32_t out = before <= 0 ? 0u : before >= 8 ? FULL_MASK : (1u << (4 * before)) - 1u;
+  return (t & ~out) | (0x55555555u & out);
+}
+
+// One column of the window; hin: the horizontal delta (0 or +1) below it. With
+// BITS the cells' two bits go to bits[k * 32].
+template <int W, bool BITS>
+__device__ __forceinline__ void band_column(const uint32_t* __restrict__ eq, uint32_t hin, uint32_t (&Pv)[W],
+                                            uint32_t (&Mv)[W], uint2* __restrict__ bits) {
+  uint32_t e[W], t[W], s[W];
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    e[k] = eq[k * 32];
+    t[k] = e[k] & Pv[k];
+  }
+  if constexpr (W == 1) {
+    s[0] = t[0] + Pv[0];
+  } else {
+    asm volatile("add.cc.u32 %0, %1, %2;" : "=r"(s[0]) : "r"(t[0]), "r"(Pv[0]));
+#pragma unroll
+    for (int k = 1; k < W - 1; ++k) asm volatile("addc.cc.u32 %0, %1, %2;" : "=r"(s[k]) : "r"(t[k]), "r"(Pv[k]));
+    asm volatile("addc.u32 %0, %1, %2;" : "=r"(s[W - 1]) : "r"(t[W - 1]), "r"(Pv[W - 1]));
+  }
+  uint32_t php = hin << 31, mhp = 0u;
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    const uint32_t pv = Pv[k], mv = Mv[k];
+    const uint32_t xv = e[k] | mv;
+    const uint32_t xh = (s[k] ^ pv) | e[k];
+    const uint32_t ph = mv | ~(xh | pv);
+    const uint32_t mh = pv & xh;
+    const uint32_t phs = __funnelshift_l(php, ph, 1), mhs = __funnelshift_l(mhp, mh, 1);
+    Pv[k] = mhs | ~(xv | phs);
+    Mv[k] = phs & xv;
+    if (BITS) {
+      const uint32_t dg = e[k] | ~(xh | mv);
+      bits[k * 32] = make_uint2(dg, e[k] | (~dg & Pv[k]));
+    }
+    php = ph;
+    mhp = mh;
+  }
+}
+
+// The candidates of list places first .. first + 31.
+template <int W>
+__device__ __forceinline__ void band_group(const TbArgs& a, uint32_t first, uint32_t* __restrict__ sm,
+                                           uint2* __restrict__ slot, uint32_t lane) {
+  BandLane c;
+  const uint32_t k0 = first + lane;
+  const uint32_t id = k0 < a.count ? a.ids[k0] : 0u;
+  bool on = k0 < a.count && tb_setup(a, id, a.results[id], 0u, c.g) == 0u;
+  c.tw = on ? (c.g.m + 31u) >> 5 : 1u;
+  c.nc = on ? c.g.c1 - c.g.a0 : 0u;
+  c.base = on ? (long long)c.g.start + c.g.c1 : 0;
+  if (!on) c.g = TbGeom{};
+  const int nc = (int)__reduce_max_sync(FULL_MASK, c.nc);
+  const int nq = (nc + 7) >> 3;
+  uint32_t* peq = sm + lane;
+  uint2* bits = reinterpret_cast<uint2*>(sm + BandMem<W>::kPeq) + lane;
+  slot += lane;
+
+  // forward: every lane starts in its first column, with the window at word 0
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    band_load<W>(a, c, peq, k, k, on);
+    peq[(5 * W + k) * 32] = 0u;
+  }
+  uint32_t Pv[W], Mv[W];
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    Pv[k] = FULL_MASK;
+    Mv[k] = 0u;
+  }
+  int below = 0;  // the value of the row below the window
+  int x = 0;      // the window's first word
+  for (int q = nq - 1; q >= 0; --q) {
+    const int want = band_first<W>(c, q >> 2);
+    if (__any_sync(FULL_MASK, want > x)) {  // at most one word per 32 columns
+      if (want > x) {
+        below += __popc(Pv[0]) - __popc(Mv[0]);
+#pragma unroll
+        for (int k = 0; k + 1 < W; ++k) {
+          Pv[k] = Pv[k + 1];
+          Mv[k] = Mv[k + 1];
+#pragma unroll
+          for (int b = 0; b < 5; ++b) peq[(b * W + k) * 32] = peq[(b * W + k + 1) * 32];
+        }
+        Pv[W - 1] = FULL_MASK;
+        Mv[W - 1] = 0u;
+        x = want;
+        band_load<W>(a, c, peq, W - 1, x + W - 1, on);
+      }
+    }
+    uint2* save = slot + (size_t)q * (W * 32);
+#pragma unroll
+    for (int k = 0; k < W; ++k) save[k * 32] = make_uint2(Pv[k], Mv[k]);
+    uint32_t t = band_text(a, c, q);
+    const uint32_t hin = x > 0 ? 1u : 0u;
+    below += 8 * (int)hin;
+#pragma unroll 1
+    for (int u = 0; u < 8; ++u) {
+      band_column<W, false>(peq + (t & 7u) * (W * 32), hin, Pv, Mv, nullptr);
+      t >>= 4;
+    }
+  }
+  // the recomputed score of the end cell must be the result's
+  int score = below - (int)(32u * c.tw - c.g.m);
+#pragma unroll
+  for (int k = 0; k < W; ++k)
+    if (x + k < (int)c.tw) score += __popc(Pv[k]) - __popc(Mv[k]);
+  if (on && score != (int)c.g.s) {
+    a.alns[id].y = kTbInconsistent;
+    on = false;
+  }
+
+  // backward: recompute 8 columns, walk through them
+  uint32_t* out = a.ops + (size_t)id * a.max_ops;
+  uint32_t i = on ? c.g.m : 0u, j1 = c.g.c1;
+  uint32_t nruns = 0, cur = 0, len = 0;
+  bool bad = false;
+  auto take = [&](uint32_t op, uint32_t count) {
+    if (len && op == cur) {
+      len += count;
+    } else {
+      if (len) {
+        if (nruns < a.max_ops) out[a.max_ops - 1u - nruns] = (len << 4) | cur;
+        ++nruns;
+      }
+      cur = op;
+      len = count;
+    }
+  };
+  for (int q = 0; q < nq && __any_sync(FULL_MASK, i > 0u); ++q) {
+    const int want = band_first<W>(c, q >> 2);
+    if (__any_sync(FULL_MASK, want < x)) {
+      if (want < x) {
+#pragma unroll
+        for (int k = W - 1; k > 0; --k)
+#pragma unroll
+          for (int b = 0; b < 5; ++b) peq[(b * W + k) * 32] = peq[(b * W + k - 1) * 32];
+        x = want;
+        band_load<W>(a, c, peq, 0, x, true);
+      }
+    }
+    const uint2* saved = slot + (size_t)q * (W * 32);
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const uint2 v = saved[k * 32];
+      Pv[k] = v.x;
+      Mv[k] = v.y;
+    }
+    uint32_t t = band_text(a, c, q);
+    const uint32_t hin = x > 0 ? 1u : 0u;
+#pragma unroll 1
+    for (int u = 7; u >= 0; --u) {  // u: columns from the end, modulo 8
+      band_column<W, true>(peq + (t & 7u) * (W * 32), hin, Pv, Mv, bits + u * (W * 32));
+      t >>= 4;
+    }
+    while (i > 0u) {
+      if (j1 <= c.g.a0) {  // only the query's bases are left
+        take(kOpI, i);
+        i = 0u;
+        break;
+      }
+      const uint32_t from_end = c.g.c1 - j1;
+      if (from_end >= 8u * (uint32_t)q + 8u) break;
+      const uint32_t bit = 32u * c.tw - c.g.m + i - 1u;
+      const int k = (int)(bit >> 5) - x;
+      if (k < 0 || k >= W) {  // outside the band: the data is inconsistent
+        bad = true;
+        break;
+      }
+      const uint2 v = bits[((from_end & 7u) * W + (uint32_t)k) * 32u];
+      const uint32_t dg = (v.x >> (bit & 31u)) & 1u, e = (v.y >> (bit & 31u)) & 1u;
+      take(dg ? (e ? kOpEq : kOpX) : (e ? kOpI : kOpD), 1u);
+      if (dg || e) --i;
+      if (dg || !e) --j1;
+    }
+    if (bad) i = 0u;
+  }
+  if (!on) return;
+  if (i > 0u) take(kOpI, i);  // the first column is reached
+  if (bad) {
+    a.alns[id].y = kTbInconsistent;
+    return;
+  }
+  if (len) {
+    if (nruns < a.max_ops) out[a.max_ops - 1u - nruns] = (len << 4) | cur;
+    ++nruns;
+  }
+  // runs were written last first at the end of the region: move them to the front
+  if (nruns <= a.max_ops) {
+    const uint32_t src = a.max_ops - nruns;
+    for (uint32_t r = 0; r < nruns; r += 8) {  // eight loads at once: the source lies behind, so none is overwritten before
+      uint32_t v[8];
+#pragma unroll
+      for (uint32_t b = 0; b < 8; ++b) v[b] = r + b < nruns ? out[src + r + b] : 0u;
+#pragma unroll
+      for (uint32_t b = 0; b < 8; ++b)
+        if (r + b < nruns) out[r + b] = v[b];
+    }
+  }
+  a.alns[id] = make_uint4(j1, nruns, c.g.s, c.g.c1 - 1u);
+}
+
+constexpr int kBandMaxWords = 15;
+constexpr int kBandWarps = 2;  // per block
+
+// Warps take 32 list places at a time from a counter; each has a slot of
+// slot_bytes for its saved states and warp_words of shared memory. Each group
+// runs with the narrowest window that holds its bands.
+template <int WMAX>
+__global__ void __launch_bounds__(32 * kBandWarps) k_tb_band(TbArgs a, unsigned long long slot_bytes, uint32_t warp_words) {
+  extern __shared__ __align__(16) uint32_t band_smem[];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  uint32_t* sm = band_smem + warp * warp_words;
+  uint2* slot = reinterpret_cast<uint2*>(a.scratch + (size_t)(blockIdx.x * kBandWarps + warp) * slot_bytes);
+  while (true) {
+    uint32_t v = 0;
+    if (lane == 0) v = atomicAdd(&a.next[0], 32u);
+    const uint32_t first = __shfl_sync(FULL_MASK, v, 0);
+    if (first >= a.count) break;
+    uint32_t w = 0;
+    if (first + lane < a.count) {
+      const uint32_t id = a.ids[first + lane];
+      TbGeom g;
+      if (tb_setup(a, id, a.results[id], 0u, g) == 0u) w = tb_window(g.s, (g.m + 31u) >> 5);
+    }
+    w = __reduce_max_sync(FULL_MASK, w);
+    if (w <= 3u) band_group<3>(a, first, sm, slot, lane);
+    else if (w <= 5u) band_group<5>(a, first, sm, slot, lane);
+    else if (WMAX == 7 || w <= 7u) band_group<7>(a, first, sm, slot, lane);
+    else if constexpr (WMAX > 7) {
+      if (w <= 9u) band_group<9>(a, first, sm, slot, lane);
+      else if (w <= 11u) band_group<11>(a, first, sm, slot, lane);
+      else if (w <= 13u) band_group<13>(a, first, sm, slot, lane);
+      else band_group<15>(a, first, sm, slot, lane);
+    }
+    __syncwarp();
+  }
+}
+
 }  // namespace myers
 
 using namespace myers;
@@ -621,6 +954,32 @@ static cudaError_t launch_tb_forward(const TbArgs& a, uint32_t cnt, int num_sms,
   return cudaGetLastError();
 }
 
+// The banded kernel over the whole list, or cudaErrorNotSupported where the
+// scratch holds too few of its slots (or a band is too wide for it).
+template <int WMAX>
+static cudaError_t launch_tb_band(const TbArgs& a, const TbState& st, uint64_t scratch_bytes, int num_sms, cudaStream_t s) {
+  // a group's window may be wider than its widest band by one word
+  const uint32_t window = st.max_band <= 3u ? 3u : st.max_band | 1u;
+  const uint32_t warp_words = window * (BandMem<WMAX>::kWords / WMAX);
+  const size_t smem = (size_t)kBandWarps * warp_words * 4;
+  cudaError_t e = cudaFuncSetAttribute(k_tb_band<WMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tb_band<WMAX>, 32 * kBandWarps, smem);
+  if (e != cudaSuccess) return e;
+  const unsigned long long slot = ((unsigned long long)(st.max_columns + 7u) >> 3) * window * 256ull;
+  const unsigned long long slots = scratch_bytes / slot;
+  unsigned long long blocks = ((unsigned long long)a.count + 32u * kBandWarps - 1u) / (32u * kBandWarps);
+  const unsigned long long full = (unsigned long long)num_sms * (per_sm > 0 ? per_sm : 1);
+  if (blocks > full) blocks = full;
+  if (slots / kBandWarps < blocks) {
+    blocks = slots / kBandWarps;
+    if (blocks < full / 4) return cudaErrorNotSupported;
+  }
+  k_tb_band<WMAX><<<(unsigned)blocks, 32 * kBandWarps, smem, s>>>(a, slot, warp_words);
+  return cudaGetLastError();
+}
+
 extern "C" int myersTraceback(myersTraceback_t* tb, const myersReference_t* ref, const qryEntry_t* d_peq,
                               uint32_t numPEQEntries, const qryInfo_t* d_qinfo, uint32_t numQueries,
                               const candInfo_t* d_cands, const resEntry_t* d_results, uint32_t numCandidates,
@@ -686,6 +1045,18 @@ extern "C" int myersTraceback(myersTraceback_t* tb, const myersReference_t* ref,
   // the last of them ends within H + max_units <= half the scratch
   const unsigned long long half_units = (tb->scratch_bytes / 2) >> kTbUnitShift;
   if (half_units <= st.max_units) return MYERS_E_CAPACITY;  // one band does not fit half the scratch
+  if (st.max_band <= (unsigned)kBandMaxWords) {
+    TbArgs ba = a;
+    ba.scratch = tb->d_scratch;
+    ba.next = tb->d_state->next[0];  // zero since the memset above
+    e = st.max_band <= 7u ? launch_tb_band<7>(ba, st, tb->scratch_bytes, tb->num_sms, s)
+                          : launch_tb_band<kBandMaxWords>(ba, st, tb->scratch_bytes, tb->num_sms, s);
+    if (e == cudaSuccess) {
+      tb->last_chunks = 1;
+      return MYERS_SUCCESS;
+    }
+    if (e != cudaErrorNotSupported) return cuda_fail(e, "k_tb_band");
+  }
   const unsigned long long H = half_units - st.max_units;
   const unsigned long long chunks = (total + H - 1ull) / H;
   const uint32_t est = (uint32_t)((unsigned long long)count * (H < total ? H : total) / total) + 1u;
