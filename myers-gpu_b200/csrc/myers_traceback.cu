@@ -8,7 +8,10 @@
 // each cell, the first of: the diagonal ('=' or 'X'), the query base alone
 // ('I'), the text base alone ('D') that is consistent with the matrix.
 //
-// Two passes per chunk of traced candidates:
+// Where the bands are at most 15 words wide (scores up to 224, or short reads)
+// and the scratch holds a slot per resident warp, one kernel recomputes the
+// band alone and walks (k_tb_band). Otherwise two passes per chunk of traced
+// candidates:
 //  * k_tb_forward: a candidate's rows are spread over L lanes of W words (W
 //    >= 8, one choice per call), a warp holding 32/S candidates in segments
 //    of S lanes. Lanes run as a systolic pipeline (lane r processes column
@@ -71,6 +74,8 @@ struct TbState {
   unsigned int next[2][2];  // per scratch half: work counters of the forward pass and the walk
   unsigned int max_band;    // widest diagonal band (words, tb_window) of a traced candidate
   unsigned int max_columns; // most columns of one
+  unsigned int bucket[256]; // candidates per band width and length (tb_bucket), for the banded kernel
+  unsigned int cursor[256];
 };
 
 struct TbArgs {
@@ -176,6 +181,18 @@ __device__ __forceinline__ uint32_t tb_window(uint32_t s, uint32_t words) {
   return w < words ? w : words;
 }
 
+// Bucket of a band of w words (windows of 15, 13, .. 1 words, or wider than 15
+// with the first) and `columns` columns (half octaves, longest first): the
+// banded kernel's warps take candidates in this order, so that its 32 lanes
+// have much the same work, the widest and longest first.
+__device__ __forceinline__ uint32_t tb_bucket(uint32_t w, uint32_t columns) {
+  const uint32_t wide = w >= 15u ? 7u : w >> 1;  // 0: one word, 7: 15
+  const uint32_t c = columns < 2u ? 2u : columns;
+  const uint32_t log2 = 31u - __clz(c);
+  const uint32_t half = 2u * log2 + (c >> (log2 - 1u) & 1u);  // 2 .. 31 for up to 65,535 columns
+  return (7u - wide) * 32u + 31u - (half < 31u ? half : 31u);
+}
+
 // Pick the candidates to trace; write the records of the others.
 __global__ void k_tb_select(TbArgs a, uint32_t* ids, unsigned long long* offs) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -212,6 +229,9 @@ __global__ void k_tb_select(TbArgs a, uint32_t* ids, unsigned long long* offs) {
         atomicMax(&a.st->max_band, b);
         atomicMax(&a.st->max_columns, c);
       }
+      const uint32_t bucket = traced ? tb_bucket(window, columns) : 0xFFFFFFFFu;
+      const uint32_t peers = __match_any_sync(FULL_MASK, bucket);
+      if (traced && (int)lane == __ffs(peers) - 1) atomicAdd(&a.st->bucket[bucket], __popc(peers));
     }
     unsigned long long incl = units;  // inclusive prefix of the units over the warp
 #pragma unroll
@@ -574,9 +594,12 @@ __global__ void __launch_bounds__(128) k_tb_walk(TbArgs a) {
 // but the saved states (W x 8 bytes per 8 columns) goes through memory, in a
 // slot per resident warp, so one launch traces everything that is traced.
 //
-// Bound by the ALU pipe. Storing the bands of a full recomputation and walking
-// them in a second kernel, a 30K-candidate call of 1,000-base reads took 3.1
-// ms; TB_FIGURES
+// Bound by the latency of a warp's chain of columns where there are few
+// candidates (one round of warps up to about 45K), else by the ALU pipe. By a
+// full recomputation, its bands stored and walked in a second kernel, a call
+// with 30K candidates of 1,000-base reads took 3.1 ms, and 150K of 100..1,000
+// bases 6.3; here 0.83 and 1.18 (1.31 and 4.0 in list order, in which one wide
+// band widens the windows of 31 others, and one long read keeps them waiting).
 template <int W>
 struct BandMem {
   static constexpr uint32_t kPeq = 6u * W * 32u;       // [base, and one that matches nothing][word][lane]
@@ -615,11 +638,10 @@ __device__ __forceinline__ void band_load(const TbArgs& a, const BandLane& c, ui
 }
 
 // The text codes of the 8 columns 8 q .. 8 q + 7 from the end, the last of them
-// first (lowest nibble), 5 for columns before the candidate's first.
-__device__ __forceinline__ uint32_t band_text(const TbArgs& a, const BandLane& c, int q) {
-  const long long b = c.base - 8ll * (q + 1);
-  const uint32_t lo = ref_load(a.ref, b >> 3, a.ref_words), hi = ref_load(a.ref, (b >> 3) + 1, a.ref_words);
-  const uint32_t t = sanitize_codes(__funnelshift_r(lo, hi, 4u * (uint32_t)(b & 7)));
+// first (lowest nibble), 5 for columns before the candidate's first, from the
+// two reference words that hold them.
+__device__ __forceinline__ uint32_t band_text(const BandLane& c, int q, uint32_t lo, uint32_t hi) {
+  const uint32_t t = sanitize_codes(__funnelshift_r(lo, hi, 4u * (uint32_t)(c.base & 7)));
   const int before = 8 * q + 8 - (int)c.nc;
   const uint32_t out = before <= 0 ? 0u : before >= 8 ? FULL_MASK : (1u << (4 * before)) - 1u;
   return (t & ~out) | (0x55555555u & out);
@@ -694,6 +716,9 @@ __device__ __forceinline__ void band_group(const TbArgs& a, uint32_t first, uint
     Pv[k] = FULL_MASK;
     Mv[k] = 0u;
   }
+  // words of the reference, loaded a block ahead
+  const long long text = c.base >> 3;  // block q starts in word text - q - 1
+  uint32_t lo = ref_load(a.ref, text - nq, a.ref_words), hi = ref_load(a.ref, text - nq + 1, a.ref_words);
   int below = 0;  // the value of the row below the window
   int x = 0;      // the window's first word
   for (int q = nq - 1; q >= 0; --q) {
@@ -717,10 +742,12 @@ __device__ __forceinline__ void band_group(const TbArgs& a, uint32_t first, uint
     uint2* save = slot + (size_t)q * (W * 32);
 #pragma unroll
     for (int k = 0; k < W; ++k) save[k * 32] = make_uint2(Pv[k], Mv[k]);
-    uint32_t t = band_text(a, c, q);
+    uint32_t t = band_text(c, q, lo, hi);
+    lo = hi;
+    hi = ref_load(a.ref, text - q + 1, a.ref_words);
     const uint32_t hin = x > 0 ? 1u : 0u;
     below += 8 * (int)hin;
-#pragma unroll 1
+#pragma unroll 2
     for (int u = 0; u < 8; ++u) {
       band_column<W, false>(peq + (t & 7u) * (W * 32), hin, Pv, Mv, nullptr);
       t >>= 4;
@@ -753,6 +780,11 @@ __device__ __forceinline__ void band_group(const TbArgs& a, uint32_t first, uint
       len = count;
     }
   };
+  uint2 ahead[W];
+#pragma unroll
+  for (int k = 0; k < W; ++k) ahead[k] = nq > 0 ? slot[k * 32] : make_uint2(0u, 0u);
+  hi = ref_load(a.ref, text, a.ref_words);
+  lo = ref_load(a.ref, text - 1, a.ref_words);
   for (int q = 0; q < nq && __any_sync(FULL_MASK, i > 0u); ++q) {
     const int want = band_first<W>(c, q >> 2);
     if (__any_sync(FULL_MASK, want < x)) {
@@ -765,16 +797,18 @@ __device__ __forceinline__ void band_group(const TbArgs& a, uint32_t first, uint
         band_load<W>(a, c, peq, 0, x, true);
       }
     }
-    const uint2* saved = slot + (size_t)q * (W * 32);
+    const uint2* saved = slot + (size_t)(q + 1 < nq ? q + 1 : q) * (W * 32);
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-      const uint2 v = saved[k * 32];
-      Pv[k] = v.x;
-      Mv[k] = v.y;
+      Pv[k] = ahead[k].x;
+      Mv[k] = ahead[k].y;
+      ahead[k] = saved[k * 32];
     }
-    uint32_t t = band_text(a, c, q);
+    uint32_t t = band_text(c, q, lo, hi);
+    hi = lo;
+    lo = ref_load(a.ref, text - q - 2, a.ref_words);
     const uint32_t hin = x > 0 ? 1u : 0u;
-#pragma unroll 1
+#pragma unroll 2
     for (int u = 7; u >= 0; --u) {  // u: columns from the end, modulo 8
       band_column<W, true>(peq + (t & 7u) * (W * 32), hin, Pv, Mv, bits + u * (W * 32));
       t >>= 4;
@@ -826,14 +860,49 @@ __device__ __forceinline__ void band_group(const TbArgs& a, uint32_t first, uint
   a.alns[id] = make_uint4(j1, nruns, c.g.s, c.g.c1 - 1u);
 }
 
+// The list in bucket order: the buckets' starts, then every place.
+__global__ void k_tb_bucket_starts(TbState* st) {
+  __shared__ unsigned int sum[256];
+  const uint32_t t = threadIdx.x;
+  const unsigned int n = st->bucket[t];
+  sum[t] = n;
+  for (uint32_t d = 1; d < 256; d <<= 1) {
+    __syncthreads();
+    const unsigned int v = t >= d ? sum[t - d] : 0u;
+    __syncthreads();
+    sum[t] += v;
+  }
+  st->cursor[t] = sum[t] - n;
+}
+
+__global__ void k_tb_bucket_fill(TbArgs a, uint32_t* __restrict__ sorted) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < a.count; base += gridDim.x * blockDim.x) {
+    const uint32_t k = base + threadIdx.x;
+    uint32_t bucket = 0xFFFFFFFFu, id = 0;
+    if (k < a.count) {
+      id = a.ids[k];
+      TbGeom g;
+      if (tb_setup(a, id, a.results[id], 0u, g) == 0u) bucket = tb_bucket(tb_window(g.s, (g.m + 31u) >> 5), g.c1 - g.a0);
+    }
+    const uint32_t peers = __match_any_sync(FULL_MASK, bucket);
+    const int leader = __ffs(peers) - 1;
+    uint32_t at = 0;
+    if (bucket < 256u && (int)lane == leader) at = atomicAdd(&a.st->cursor[bucket], __popc(peers));
+    at = __shfl_sync(FULL_MASK, at, leader);
+    if (bucket < 256u) sorted[at + __popc(peers & ((1u << lane) - 1u))] = id;
+  }
+}
+
 constexpr int kBandMaxWords = 15;
 constexpr int kBandWarps = 2;  // per block
 
-// Warps take 32 list places at a time from a counter; each has a slot of
-// slot_bytes for its saved states and warp_words of shared memory. Each group
-// runs with the narrowest window that holds its bands.
+// Warps take 32 list places at a time from the counter a.next[0], up to a.count;
+// each has a slot of slot_bytes for its saved states and warp_words of shared
+// memory. Each group runs with the narrowest window that holds its bands.
 template <int WMAX>
-__global__ void __launch_bounds__(32 * kBandWarps) k_tb_band(TbArgs a, unsigned long long slot_bytes, uint32_t warp_words) {
+__global__ void __launch_bounds__(32 * kBandWarps, WMAX <= 7 ? 8 : 4)
+    k_tb_band(TbArgs a, unsigned long long slot_bytes, uint32_t warp_words) {
   extern __shared__ __align__(16) uint32_t band_smem[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   uint32_t* sm = band_smem + warp * warp_words;
@@ -850,10 +919,11 @@ __global__ void __launch_bounds__(32 * kBandWarps) k_tb_band(TbArgs a, unsigned 
       if (tb_setup(a, id, a.results[id], 0u, g) == 0u) w = tb_window(g.s, (g.m + 31u) >> 5);
     }
     w = __reduce_max_sync(FULL_MASK, w);
-    if (w <= 3u) band_group<3>(a, first, sm, slot, lane);
-    else if (w <= 5u) band_group<5>(a, first, sm, slot, lane);
-    else if (WMAX == 7 || w <= 7u) band_group<7>(a, first, sm, slot, lane);
-    else if constexpr (WMAX > 7) {
+    if constexpr (WMAX <= 7) {
+      if (w <= 3u) band_group<3>(a, first, sm, slot, lane);
+      else if (w <= 5u) band_group<5>(a, first, sm, slot, lane);
+      else band_group<7>(a, first, sm, slot, lane);
+    } else {
       if (w <= 9u) band_group<9>(a, first, sm, slot, lane);
       else if (w <= 11u) band_group<11>(a, first, sm, slot, lane);
       else if (w <= 13u) band_group<13>(a, first, sm, slot, lane);
@@ -954,30 +1024,84 @@ static cudaError_t launch_tb_forward(const TbArgs& a, uint32_t cnt, int num_sms,
   return cudaGetLastError();
 }
 
-// The banded kernel over the whole list, or cudaErrorNotSupported where the
-// scratch holds too few of its slots (or a band is too wide for it).
+// The banded kernel's launch over a.ids[0 .. a.count - 1], bands of at most `band`
+// words: its grid and what each warp needs. blocks is 0 where `bytes` of scratch
+// hold the slots of too few warps.
+struct BandLaunch {
+  uint32_t blocks, warp_words;
+  unsigned long long slot;
+  size_t smem;
+};
+
 template <int WMAX>
-static cudaError_t launch_tb_band(const TbArgs& a, const TbState& st, uint64_t scratch_bytes, int num_sms, cudaStream_t s) {
+static cudaError_t plan_tb_band(BandLaunch& l, uint32_t count, uint32_t band, uint32_t columns, uint64_t bytes, int num_sms) {
   // a group's window may be wider than its widest band by one word
-  const uint32_t window = st.max_band <= 3u ? 3u : st.max_band | 1u;
-  const uint32_t warp_words = window * (BandMem<WMAX>::kWords / WMAX);
-  const size_t smem = (size_t)kBandWarps * warp_words * 4;
-  cudaError_t e = cudaFuncSetAttribute(k_tb_band<WMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  const uint32_t window = WMAX > 7 && band < 9u ? 9u : band <= 3u ? 3u : band | 1u;
+  l.warp_words = window * (BandMem<WMAX>::kWords / WMAX);
+  l.smem = (size_t)kBandWarps * l.warp_words * 4;
+  cudaError_t e = cudaFuncSetAttribute(k_tb_band<WMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tb_band<WMAX>, 32 * kBandWarps, smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tb_band<WMAX>, 32 * kBandWarps, l.smem);
   if (e != cudaSuccess) return e;
-  const unsigned long long slot = ((unsigned long long)(st.max_columns + 7u) >> 3) * window * 256ull;
-  const unsigned long long slots = scratch_bytes / slot;
-  unsigned long long blocks = ((unsigned long long)a.count + 32u * kBandWarps - 1u) / (32u * kBandWarps);
-  const unsigned long long full = (unsigned long long)num_sms * (per_sm > 0 ? per_sm : 1);
+  l.slot = ((unsigned long long)(columns + 7u) >> 3) * window * 256ull;
+  const unsigned long long slots = bytes / l.slot, full = (unsigned long long)num_sms * (per_sm > 0 ? per_sm : 1);
+  unsigned long long blocks = ((unsigned long long)count + 32u * kBandWarps - 1u) / (32u * kBandWarps);
   if (blocks > full) blocks = full;
-  if (slots / kBandWarps < blocks) {
-    blocks = slots / kBandWarps;
-    if (blocks < full / 4) return cudaErrorNotSupported;
+  if (slots / kBandWarps < blocks) blocks = slots / kBandWarps < full / 4 ? 0 : slots / kBandWarps;
+  l.blocks = (uint32_t)blocks;
+  return cudaSuccess;
+}
+
+// Trace the whole list with the banded kernel: in bucket order, bands of more
+// than 7 words on the walk's stream beside the others. False in `done` where a
+// band is too wide or the scratch too small for it.
+static int trace_bands(myersTraceback_t* tb, const TbArgs& a, const TbState& st, cudaStream_t s, bool& done) {
+  done = false;
+  if (st.max_band > (unsigned)kBandMaxWords) return MYERS_SUCCESS;
+  uint32_t wide = 0;  // windows of 9 words or more come first
+  for (int b = 0; b < 4 * 32; ++b) wide += st.bucket[b];
+  const uint32_t narrow = a.count - wide;
+  const uint64_t half = (tb->scratch_bytes / 2) & ~255ull;
+  BandLaunch lw{}, ln{};
+  cudaError_t e = cudaSuccess;
+  if (wide) e = plan_tb_band<kBandMaxWords>(lw, wide, st.max_band, st.max_columns, half, tb->num_sms);
+  if (e == cudaSuccess && narrow)
+    e = plan_tb_band<7>(ln, narrow, st.max_band < 7u ? st.max_band : 7u, st.max_columns, half, tb->num_sms);
+  if (e != cudaSuccess) return cuda_fail(e, "k_tb_band");
+  if ((wide && lw.blocks == 0) || (narrow && ln.blocks == 0)) return MYERS_SUCCESS;
+  // the offsets of the band stores are not needed here: their array takes the sorted list
+  uint32_t* sorted = reinterpret_cast<uint32_t*>(tb->d_offs);
+  k_tb_bucket_starts<<<1, 256, 0, s>>>(tb->d_state);
+  uint32_t blocks = (a.count + 255u) / 256u;
+  if (blocks > (uint32_t)tb->num_sms * 8u) blocks = (uint32_t)tb->num_sms * 8u;
+  k_tb_bucket_fill<<<blocks, 256, 0, s>>>(a, sorted);
+  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_tb_bucket");
+  if (wide) {
+    TbArgs w = a;
+    w.ids = sorted;
+    w.count = wide;
+    w.scratch = tb->d_scratch;
+    w.next = tb->d_state->next[0];  // both counters are zero since the state was cleared
+    if ((e = cudaEventRecord(tb->fwd_done[0], s)) != cudaSuccess ||
+        (e = cudaStreamWaitEvent(tb->walk_stream, tb->fwd_done[0], 0)) != cudaSuccess)
+      return cuda_fail(e, "event");
+    k_tb_band<kBandMaxWords><<<lw.blocks, 32 * kBandWarps, lw.smem, tb->walk_stream>>>(w, lw.slot, lw.warp_words);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_tb_band");
+    if ((e = cudaEventRecord(tb->walk_done[0], tb->walk_stream)) != cudaSuccess) return cuda_fail(e, "event");
   }
-  k_tb_band<WMAX><<<(unsigned)blocks, 32 * kBandWarps, smem, s>>>(a, slot, warp_words);
-  return cudaGetLastError();
+  if (narrow) {
+    TbArgs n = a;
+    n.ids = sorted + wide;
+    n.count = narrow;
+    n.scratch = tb->d_scratch + half;
+    n.next = tb->d_state->next[1];
+    k_tb_band<7><<<ln.blocks, 32 * kBandWarps, ln.smem, s>>>(n, ln.slot, ln.warp_words);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_tb_band");
+  }
+  // the caller's stream resumes after both
+  if (wide && (e = cudaStreamWaitEvent(s, tb->walk_done[0], 0)) != cudaSuccess) return cuda_fail(e, "wait");
+  done = true;
+  return MYERS_SUCCESS;
 }
 
 extern "C" int myersTraceback(myersTraceback_t* tb, const myersReference_t* ref, const qryEntry_t* d_peq,
@@ -1045,17 +1169,14 @@ extern "C" int myersTraceback(myersTraceback_t* tb, const myersReference_t* ref,
   // the last of them ends within H + max_units <= half the scratch
   const unsigned long long half_units = (tb->scratch_bytes / 2) >> kTbUnitShift;
   if (half_units <= st.max_units) return MYERS_E_CAPACITY;  // one band does not fit half the scratch
-  if (st.max_band <= (unsigned)kBandMaxWords) {
-    TbArgs ba = a;
-    ba.scratch = tb->d_scratch;
-    ba.next = tb->d_state->next[0];  // zero since the memset above
-    e = st.max_band <= 7u ? launch_tb_band<7>(ba, st, tb->scratch_bytes, tb->num_sms, s)
-                          : launch_tb_band<kBandMaxWords>(ba, st, tb->scratch_bytes, tb->num_sms, s);
-    if (e == cudaSuccess) {
+  {
+    bool done = false;
+    const int bs = trace_bands(tb, a, st, s, done);
+    if (bs != MYERS_SUCCESS) return bs;
+    if (done) {
       tb->last_chunks = 1;
       return MYERS_SUCCESS;
     }
-    if (e != cudaErrorNotSupported) return cuda_fail(e, "k_tb_band");
   }
   const unsigned long long H = half_units - st.max_units;
   const unsigned long long chunks = (total + H - 1ull) / H;
