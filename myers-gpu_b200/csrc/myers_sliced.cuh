@@ -311,7 +311,11 @@ __device__ __forceinline__ void run_columns(const DevInputs& in, const Tile& t, 
   const WarpMem w = warp_mem<K>(threadIdx.x >> 5);
   const uint32_t one = c_one, mone = c_mone;
 
-  uint32_t q0[R], q1[R], q2[GEN ? R : 1], Pv[R], Mv[R];
+  // With many rows Pv - Mv is kept instead of formed anew: 1,000-base reads 12.8
+  // -> 12.5 ms per 660K candidates, 950 bases 12.0 -> 11.3 (no gain on fewer
+  // rows, a loss on chains of warps).
+  constexpr bool kKeepV = !K::kChain && R > 24;
+  uint32_t q0[R], q1[R], q2[GEN ? R : 1], Pv[R], Mv[R], V[kKeepV ? R : 1];
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int at = lane * K::kStride + i;
@@ -320,6 +324,7 @@ __device__ __forceinline__ void run_columns(const DevInputs& in, const Tile& t, 
     if (GEN) q2[i] = w.buf[64 * K::kStride + at];
     Pv[i] = 0xFFFFFFFFu;
     Mv[i] = 0u;
+    if (kKeepV) V[i] = 0xFFFFFFFFu;
   }
   __syncwarp();
   // Rings: 64 text columns per group; 64 columns of the last row per group,
@@ -390,15 +395,16 @@ __device__ __forceinline__ void run_columns(const DevInputs& in, const Tile& t, 
           x = lop3<kA | (kB ^ kC)>(x, q1[i], tx.y);
           const uint32_t N = lop3<kA & ~kB & ~kC>(x, Mv[i], M);
           const uint32_t m2 = lop3<kA & ~kB>(Pv[i], N, N);
-          const uint32_t h2 = mad(mad(Mv[i], mone, Pv[i]), mone, N);
+          const uint32_t h2 = mad(kKeepV ? V[i] : mad(Mv[i], mone, Pv[i]), mone, N);
           const uint32_t p2 = mad(m2, one, h2);
           const uint32_t mv = lop3<kA & ~kB>(P, N, N);
-          const uint32_t pv = mad(mv, one, mad(H, mone, N));
+          const uint32_t v2 = mad(H, mone, N), pv = mad(mv, one, v2);
           P = p2;
           M = m2;
           H = h2;
           Pv[i] = pv;
           Mv[i] = mv;
+          if (kKeepV) V[i] = v2;
           if (i == 0) {  // candidates that skip this row pass the delta on
             P = lop3<(kA & kC) | (kB & ~kC)>(Pin, P, pm);
             M = lop3<(kA & kC) | (kB & ~kC)>(Min, M, pm);
@@ -587,8 +593,7 @@ __device__ __forceinline__ void run_tile(const DevInputs& in, const Tile& t, int
 // A block's warps (groups of nw warps in a chain class) take tiles from the
 // counters of the class's shapes, in the plan's order: the longest tiles
 // first. The first tile of every group of the first shape is its place in the
-// grid, so that a launch of few tiles spreads over the SMs. With st ==
-// nullptr there is one shape, candidates 0..count-1.
+// grid. With st == nullptr there is one shape, candidates 0..count-1.
 template <class K>
 __global__ void __launch_bounds__(K::kThreads, K::kBlocks)
     k_sliced(const __grid_constant__ DevInputs in, const uint32_t* __restrict__ ids, BucketState* st,
@@ -610,6 +615,25 @@ __global__ void __launch_bounds__(K::kThreads, K::kBlocks)
     lut[x] = make_int2((int)((uint32_t)least << 16) + at, (int)((uint32_t)sum << 16) + 4);
   }
   __syncthreads();
+  uint32_t blocks = gridDim.x;
+  if constexpr (!K::kChain) {
+    // Only as many blocks as the class has tiles for stay, so that those of the
+    // other classes find room beside them (300K reads of 35..301 bases, three
+    // classes of one round or less: 0.49 -> 0.43 ms).
+    __shared__ uint32_t s_tiles;
+    if (threadIdx.x == 0) s_tiles = 0u;
+    __syncthreads();
+    uint32_t tiles = 0;
+    for (uint32_t c = c0 + threadIdx.x; c < c1; c += K::kThreads) {
+      const Shape s = plan.shape[c];
+      const uint32_t per = 32u << (5 - s.L);
+      if (K::has(s)) tiles += ((st != nullptr ? st->count[c] : count) + per - 1u) / per;
+    }
+    if (tiles) atomicAdd(&s_tiles, tiles);
+    __syncthreads();
+    blocks = min(blocks, (s_tiles + K::kWarps - 1u) / K::kWarps);
+    if (blockIdx.x >= blocks) return;
+  }
   int nw_before = 0;
   bool placed = false;
   Tile t;
@@ -638,13 +662,13 @@ __global__ void __launch_bounds__(K::kThreads, K::kBlocks)
       if (t.nw != nw_before && nw_before != 0) __syncthreads();  // the groups' shares of shared memory change hands
       nw_before = t.nw;
     }
-    const uint32_t placed_tiles = placed ? 0u : gridDim.x * ngroups;
+    const uint32_t placed_tiles = placed ? 0u : blocks * ngroups;
     bool place = !placed;
     placed = true;
     while (true) {
       uint32_t i = 0;
       if (place) {
-        i = (uint32_t)t.group * gridDim.x + blockIdx.x;
+        i = blockIdx.x * ngroups + (uint32_t)t.group;
         place = false;
       } else {
         if (lane == 0 && t.wg == 0) i = placed_tiles + atomicAdd(next, 1u);
