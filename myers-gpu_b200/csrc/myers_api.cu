@@ -295,23 +295,8 @@ static bool small_batch(uint64_t n) {
   return n > 0 && n < threshold;
 }
 
-// Whether a batch of n candidates whose lengths are flagged in present_m takes
-// bit-sliced shapes (myers_sliced.cuh) for its reads of kSlicedMinRows..
-// kSlicedMaxRows bases. A tile of theirs is 32 candidates or more on one warp
-// (on two to eight warps beyond 1,024 bases), so a batch has to fill the
-// device with such tiles. Measured, word-parallel against bit-sliced:
-//  * one length, which ends with whole rounds of tiles: 1,000 bases 33K
-//    candidates (0.87 of a round) 0.97 -> 0.85 ms, 330K 8.8 -> 6.6; 400 bases
-//    330K 1.50 -> 1.22; 100 bases 330K (1.1 rounds) 0.159 -> 0.152, 1.1M 0.446 ->
-//    0.386; 3,000 bases 11K (1.16 rounds) 3.20 -> 3.44, 44K 11.7 -> 8.5; 8,000
-//    bases 4.4K (0.93) 8.6 -> 6.0;
-//  * mixed lengths, where a round of the longest tiles comes on top: 100..1,000
-//    bases 88K 0.76 -> 0.97, 220K 1.73 -> 1.48; 1,000..10,000 bases 15K 10.9 ->
-//    11.7, 40K 25.9 -> 18.4;
-//  * the plain path's one-lane shapes of more than 16 words, and its launch per
-//    shape, need as many candidates: 1,000 bases 3.3K 0.67 -> 0.54; 35..301
-//    bases 5K 0.21 -> 0.19, 300K 0.58 -> 0.43.
-// MYERS_SLICED=0 turns the shapes off, 1 takes them for every batch.
+// MYERS_SLICED=0 turns the bit-sliced shapes off; 1 takes them for every batch, 2
+// and 3 spread once and twice.
 static int sliced_force() {
   static const int force = [] {
     const char* env = getenv("MYERS_SLICED");
@@ -319,29 +304,48 @@ static int sliced_force() {
   }();
   return force;
 }
-// Whether a batch of n candidates may take them at all: its lengths have to be
-// listed only then.
-static bool sliced_possible(uint64_t n) { return sliced_force() >= 0 ? sliced_force() > 0 : n >= 4096; }
-static bool sliced_batch(const uint8_t* present_m, bool batched, uint64_t n) {
-  if (!sliced_possible(n)) return false;
-  if (sliced_force() > 0) return true;
-  uint32_t lo = 0, hi = 0;
-  for (uint32_t m = kSlicedMinRows; m <= kSlicedMaxRows; ++m)
-    if (present_m[m]) {
-      if (lo == 0) lo = m;
-      hi = m;
-    }
-  if (hi == 0) return false;
+
+// Whether a batch of n candidates of queries of lo..hi bases takes bit-sliced
+// shapes (myers_sliced.cuh) for those of kSlicedMinRows..kSlicedMaxRows bases,
+// and how far it spreads them. A tile of theirs is 32 candidates or more on one
+// warp (on two to eight warps beyond 1,024 bases), so a batch has to fill the
+// device with such tiles. Measured, word-parallel against bit-sliced:
+//  * one length, which ends with whole rounds of tiles: 1,000 bases 33K
+//    candidates (0.87 of a round) 0.98 -> 0.82 ms, 660K 17.3 -> 12.5; 400 bases
+//    330K 1.50 -> 1.17; 100 bases 330K (1.1 rounds) 0.159 -> 0.152, 1.1M 0.446 ->
+//    0.38; 3,000 bases 11K (1.16 rounds) 3.1 -> 3.6, 44K 11.7 -> 8.5; 8,000
+//    bases 4.4K (0.93) 8.6 -> 6.0;
+//  * mixed lengths, where a round of the longest tiles comes on top: 100..1,000
+//    bases 33K 0.46 -> 0.58, 110K (2.9 rounds of the longest) 0.93 -> 0.89, 220K
+//    1.73 -> 1.35; 1,000..10,000 bases 15K 10.9 -> 11.2, 40K 25.9 -> 18.6;
+//  * the plain path's one-lane shapes of more than 16 words, and its launch per
+//    shape, need as many candidates: 1,000 bases 3.3K 0.67 -> 0.52; 35..301
+//    bases 5K 0.24 -> 0.13, 50K 0.42 -> 0.16 (spread twice; 0.26 unspread).
+static bool sliced_batch(Lengths len, bool batched, uint64_t n, uint32_t& spread) {
+  spread = 0;
+  if (sliced_force() == 0 || len.hi < kSlicedMinRows || len.lo > kSlicedMaxRows) return false;
+  if (sliced_force() < 0 && n < 4096) return false;
+  const uint32_t lo = len.lo < kSlicedMinRows ? kSlicedMinRows : len.lo;
+  const uint32_t hi = len.hi > kSlicedMaxRows ? kSlicedMaxRows : len.hi;
   int lg, R, lg_lo, R_lo;
-  const bool one = sliced_shape(lo, &lg_lo, &R_lo) == sliced_shape(hi, &lg, &R);
+  const bool one = sliced_shape(lo, 0, &lg_lo, &R_lo) == sliced_shape(hi, 0, &lg, &R);
   const uint64_t per = 32u << (lg < 5 ? 5 - lg : 0), nw = lg > 5 ? 1u << (lg - 5) : 1u;
   const uint64_t round = 148u * (uint64_t)kSlicedWarps[sliced_class(Shape{kSlicedVariant, (uint8_t)lg, (uint8_t)R, 0})] / nw;
   const uint64_t tiles = (n + per - 1) / per;
-  if (!one) return tiles >= 4 * round || (!batched && hi <= 1024);
+  if (sliced_force() > 0) {
+    spread = (uint32_t)sliced_force() - 1u;
+    return true;
+  }
+  // Reads of many short lengths are a round of every class of shapes: doubled
+  // tiles shorten them while they stay within some rounds (300K reads of 35..301
+  // bases 0.41 -> 0.36 ms, 150K 0.34 -> 0.26).
+  if (!one && lg < 5)
+    while (spread < 2 && (tiles << (spread + 1)) <= kSpreadRounds * round) ++spread;
+  if (!one) return 4 * tiles >= 11 * round || (!batched && hi <= 1024);
   const uint64_t rounds = (tiles + round - 1) / round;
   if (!batched && hi > 512 && hi <= 1024 && rounds <= 1) return true;
   if (hi <= 512 && rounds < 2) return false;
-  return rounds >= 4 || 4 * tiles >= 3 * rounds * round;
+  return rounds >= 4 || 10 * tiles >= 7 * rounds * round;
 }
 
 // lane_words > 0 asks for latency-oriented shapes: a query of more than
@@ -403,7 +407,7 @@ static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words = 0, bool 
 // Build the plan for the word counts flagged in `present` (size kMaxWords+1).
 // Uses fixed-size stack arrays only: no allocation on the send path.
 int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, uint64_t n,
-                      uint64_t reads, const uint8_t* present_m, bool bucketed, uint64_t sliced_n) {
+                      uint64_t reads, Lengths lengths, bool bucketed, uint64_t sliced_n) {
   memset(&t, 0, sizeof(t));
   memset(t.cfg_of_words, kNoCfg, sizeof(t.cfg_of_words));
   memset(t.cfg_of_sliced, kNoCfg, sizeof(t.cfg_of_sliced));
@@ -421,7 +425,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   // Bit-sliced shapes: for the word counts without an override, every length
   // of a word count that is present (lengths the caller did not announce but
   // whose word count occurs are admitted, as by the word-parallel shapes).
-  const bool sliced = present_m != nullptr && lane_words == 0 && sliced_batch(present_m, batched, sliced_n ? sliced_n : n);
+  const bool sliced = lane_words == 0 && sliced_batch(lengths, batched, sliced_n ? sliced_n : n, t.spread);
   uint8_t sliced_words[kMaxWords + 1];
   memset(sliced_words, 0, sizeof(sliced_words));
   uint32_t sliced_rows[kSlicedShapes];  // longest length of each bit-sliced shape
@@ -431,8 +435,15 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     for (uint32_t w = kSlicedMinRows / 32 + 1; w <= kSlicedMaxRows / 32; ++w)
       sliced_words[w] = present[w] && !g_override[batched ? 1 : 0][w].set;
   }
-  bool alone = sliced && !bucketed;  // every length present has the same bit-sliced shape
+  // every length that can occur has the same bit-sliced shape (a longer length
+  // never has a smaller one)
+  bool alone = sliced && !bucketed && lengths.lo >= kSlicedMinRows && lengths.hi <= kSlicedMaxRows;
   int alone_shape = -1;
+  if (alone) {
+    int lg, R;
+    alone_shape = sliced_shape(lengths.lo, t.spread, &lg, &R);
+    alone = alone_shape == sliced_shape(lengths.hi, t.spread, &lg, &R);
+  }
   uint32_t w_lo = 0, w_hi = 0;
   for (uint32_t w = 1; w <= kMaxWords; ++w) {
     if (!present[w]) continue;
@@ -442,11 +453,8 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
       t.cfg_of_words[w] = kSlicedCfg;
       for (uint32_t m = 32 * (w - 1) + 1; m <= 32 * w; ++m) {
         int lg, R;
-        const int i = sliced_shape(m, &lg, &R);
+        const int i = sliced_shape(m, t.spread, &lg, &R);
         sliced_rows[i] = m;
-        if (!present_m[m]) continue;
-        if (alone_shape >= 0 && alone_shape != i) alone = false;
-        alone_shape = i;
       }
       continue;
     }
@@ -468,12 +476,11 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     if (w > max_words[found]) max_words[found] = w;
     cfg_of[w] = (int16_t)found;
   }
-  alone = alone && alone_shape >= 0;
   for (int i = 0; i < kSlicedShapes; ++i) {
     if (sliced_rows[i] == 0 || (alone && i != alone_shape)) continue;
     if (nshapes == kMaxCfg) return MYERS_E_QUERY_TOO_LONG;
     int lg, R;
-    sliced_shape(sliced_rows[i], &lg, &R);
+    sliced_shape(sliced_rows[i], t.spread, &lg, &R);
     shapes[nshapes] = Shape{kSlicedVariant, (uint8_t)lg, (uint8_t)R, 0};
     max_words[nshapes] = sliced_rows[i];
     ++nshapes;
@@ -526,7 +533,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     if (group[order[r]] == 1) {
       ++t.num_sliced;
       int lg, R;
-      t.cfg_of_sliced[sliced_shape(max_words[order[r]], &lg, &R)] = (uint8_t)r;
+      t.cfg_of_sliced[sliced_shape(max_words[order[r]], t.spread, &lg, &R)] = (uint8_t)r;
     }
   }
   for (uint32_t w = 1; w <= kMaxWords; ++w)
@@ -642,18 +649,23 @@ int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* presen
   uint8_t w1[kMaxWords + 1], w2[kMaxWords + 1];
   memset(w1, 0, sizeof(w1));
   memset(w2, 0, sizeof(w2));
-  std::vector<uint8_t> m1(kMaxWords * 32 + 1, 0), m2(kMaxWords * 32 + 1, 0);
+  Lengths m1, m2;
   for (uint32_t m = 1; m <= kMaxWords * 32; ++m) {
     if (!present_m[m]) continue;
     const uint32_t r = host_prefix_rows(m, cutoff, mult);
-    m1[r] = 1;
     w1[(r + 31) / 32] = 1;
-    if (r < m) m2[m] = w2[(m + 31) / 32] = 1;
+    if (m1.lo == 0) m1.lo = r;  // rows grow with the length
+    m1.hi = r;
+    if (r < m) {
+      w2[(m + 31) / 32] = 1;
+      if (m2.lo == 0) m2.lo = m;
+      m2.hi = m;
+    }
   }
   // the second pass holds the candidates that survived, mostly one per read
   auto both = [&](bool bucketed) {
-    const int st = build_plan(plan, w1, batched, 0, n, 0, m1.data(), bucketed);
-    return st != MYERS_SUCCESS ? st : build_plan(plan2, w2, batched, 0, n, n, m2.data(), bucketed, n / 8);
+    const int st = build_plan(plan, w1, batched, 0, n, 0, m1, bucketed);
+    return st != MYERS_SUCCESS ? st : build_plan(plan2, w2, batched, 0, n, n, m2, bucketed, n / 8);
   };
   int st = both(batched);
   // more than one shape in either pass: both are classified
@@ -848,10 +860,7 @@ static int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, i
   if (maxSize > kMaxWords * 32) maxSize = kMaxWords * 32;
   const uint32_t wlo = minSize ? (minSize + 31) / 32 : 1, whi = (maxSize + 31) / 32;
   for (uint32_t w = wlo; w <= whi; ++w) present[w] = 1;
-  if (!sliced_possible(n)) return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, n, reads);
-  std::vector<uint8_t> present_m(kMaxWords * 32 + 1, 0);
-  for (uint32_t m = minSize ? minSize : 1; m <= maxSize; ++m) present_m[m] = 1;
-  return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, n, reads, present_m.data());
+  return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, n, reads, Lengths{minSize ? minSize : 1, maxSize});
 }
 
 extern "C" int myersVerifyAsync(myersContext_t* ctx, const myersReference_t* ref, const qryEntry_t* d_peq,
@@ -1104,7 +1113,7 @@ struct Buffer {
   int last_status;
   bool pending;
   std::vector<uint8_t> present;    // word counts of the last send
-  std::vector<uint8_t> present_m;  // query lengths of the last send
+  std::vector<uint8_t> present_m;  // query lengths of the last send (cut-off only)
   PlanTable plan, plan2;
   bool plan_valid;
   int plan_path;
@@ -1216,7 +1225,6 @@ extern "C" int myersInit(void*** myersBuffer, uint32_t numBuffers, const char* r
     const char* g = getenv("MYERS_GRAPHS");
     b->use_graphs = !(g && strcmp(g, "0") == 0);
     b->present.assign(kMaxWords + 1, 0);
-    b->present_m.assign(kMaxWords * 32 + 1, 0);
     bufs[i] = b;
     st = buffer_alloc(b);
     if (st != MYERS_SUCCESS) {
@@ -1247,27 +1255,32 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
   CU(cudaSetDevice(b->device));
   // O(queries) host pass: the word counts present pick the shapes
   std::vector<uint8_t>& present = b->present;
-  std::vector<uint8_t>& pm = b->present_m;
   const bool two_pass = b->cutoff >= 0.0f;
-  const bool lengths = two_pass || sliced_possible(numCandidates);  // ... and the lengths, where they can matter
+  Lengths lengths;
   std::fill(present.begin(), present.end(), 0);
-  if (lengths) std::fill(pm.begin(), pm.end(), 0);
   for (uint32_t q = 0; q < numQueries; ++q) {
     const uint32_t m = b->h_qinfo[q].size;
     if (m == 0 || m > kMaxWords * 32) continue;  // longer: flagged on the device
     present[(m + 31) / 32] = 1;
-    if (lengths) pm[m] = 1;
+    if (lengths.lo == 0 || m < lengths.lo) lengths.lo = m;
+    if (m > lengths.hi) lengths.hi = m;
   }
   PlanTable& plan = b->plan;
   int st;
   {
     NvtxRange plan_range("myers: send: shape plan");
     if (two_pass) {
+      std::vector<uint8_t>& pm = b->present_m;
+      pm.assign(kMaxWords * 32 + 1, 0);
+      for (uint32_t q = 0; q < numQueries; ++q) {
+        const uint32_t m = b->h_qinfo[q].size;
+        if (m > 0 && m <= kMaxWords * 32) pm[m] = 1;
+      }
       st = cutoff_plans(plan, b->plan2, pm.data(), b->cutoff, cutoff_prefix_mult(), b->path == MYERS_PATH_BATCHED,
                         numCandidates);
     } else {
       st = build_plan(plan, present.data(), b->path == MYERS_PATH_BATCHED, 0, numCandidates, numQueries,
-                      lengths ? pm.data() : nullptr);
+                      lengths);
     }
   }
   if (st != MYERS_SUCCESS) return b->last_status = st;

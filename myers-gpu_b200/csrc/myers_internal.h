@@ -85,17 +85,20 @@ constexpr uint8_t kNoCfg = 0xFF;
 // Bit-sliced shapes (myers_sliced.cuh): Shape{kSlicedVariant, log2 of the lanes
 // per group of 32 candidates, rows per lane}. The lanes are the smallest of
 // 8, 16, .. 256 that need at most 32 rows each (40 with 256 lanes, in steps of
-// two above 32).
+// two above 32); `spread` doubles the lanes that many times, up to the warp's
+// 32 and as long as a lane keeps 8 rows, so that a batch of short reads fills
+// more warps.
 constexpr uint8_t kSlicedVariant = 0xFE;
 constexpr uint8_t kSlicedCfg = 0xFE;    // cfg_of_words: look in cfg_of_sliced
 constexpr uint32_t kSlicedMinRows = 65, kSlicedMaxRows = 10240;
-constexpr int kSlicedMinLg = 3, kSlicedMaxLg = 8, kSlicedMinR = 9, kSlicedMaxR = 40;
+constexpr int kSlicedMinLg = 3, kSlicedMaxLg = 8, kSlicedMinR = 8, kSlicedMaxR = 40;
 constexpr int kSlicedShapes = (kSlicedMaxLg - kSlicedMinLg + 1) * (kSlicedMaxR - kSlicedMinR + 1);
 
 // Index of the bit-sliced shape of m rows (kSlicedMinRows..kSlicedMaxRows).
-__host__ __device__ inline int sliced_shape(uint32_t m, int* lg, int* R) {
+__host__ __device__ inline int sliced_shape(uint32_t m, uint32_t spread, int* lg, int* R) {
   int g = kSlicedMinLg;
   while (g < kSlicedMaxLg && m > (32u << g)) ++g;
+  for (; spread > 0 && g < 5 && m > (7u << (g + 1)); --spread) ++g;
   int r = (int)((m + (1u << g) - 1u) >> g);
   if (r > 32) r += r & 1;
   *lg = g;
@@ -114,6 +117,7 @@ struct PlanTable {
   uint32_t num_cfg;
   uint32_t num_batched;
   uint32_t num_sliced;
+  uint32_t spread;     // of the bit-sliced shapes
   uint32_t row_min, row_limit;  // one bit-sliced shape without bucketing: the queries it admits (else 0, 0)
   Shape shape[kMaxCfg];
 };
@@ -124,7 +128,7 @@ __host__ __device__ inline uint32_t plan_cfg(const PlanTable& plan, uint32_t m) 
   if (c != kSlicedCfg) return c;
   if (m < kSlicedMinRows || m > kSlicedMaxRows) return kNoCfg;
   int lg, R;
-  return plan.cfg_of_sliced[sliced_shape(m, &lg, &R)];
+  return plan.cfg_of_sliced[sliced_shape(m, plan.spread, &lg, &R)];
 }
 
 // Device-computed layout of the bucketed candidate list.
@@ -227,6 +231,7 @@ cudaError_t launch_batched(const DevInputs& in, const uint32_t* d_ids, const Pla
 // The bit-sliced kernels (myers_sliced.cuh), one per class of shapes.
 constexpr int kSlicedClasses = 4;
 inline int sliced_class(const Shape& s) { return s.L > 5 ? 3 : s.W <= 16 ? 0 : s.W <= 24 ? 1 : 2; }
+constexpr uint64_t kSpreadRounds = 6;           // tiles of short reads are doubled up to so many rounds
 constexpr int kSlicedWarps[kSlicedClasses] = {16, 12, 8, 8};  // warps per SM
 // A launch over the class's shapes among shapes c0..c1-1 of the plan, their lists
 // in d_state (whose next counters start at zero); with d_state == nullptr over
@@ -283,13 +288,16 @@ cudaError_t launch_lop3_probe(uint32_t* d_out, int blocks, int threads, int iter
 // n: the batch's candidates, which picks the batched path's table for large
 // batches at kLargeBatchCandidates or more.
 // reads: how many reads the n candidates come from (0: unknown).
-// present_m: flags each query length 1..kMaxWords * 32 that can occur; with
-// it, large batches take bit-sliced shapes.
+// lengths: the shortest and longest query that can occur; with them, large
+// batches take bit-sliced shapes.
 // bucketed: the candidates will be classified by the plan in any case, so it
 // names every shape of the word counts present.
 // sliced_n: candidates expected, where they are not n (the cut-off's second pass).
+struct Lengths {
+  uint32_t lo = 0, hi = 0;  // 0, 0: unknown
+};
 int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words = 0, uint64_t n = 0,
-               uint64_t reads = 0, const uint8_t* present_m = nullptr, bool bucketed = false, uint64_t sliced_n = 0);
+               uint64_t reads = 0, Lengths lengths = {}, bool bucketed = false, uint64_t sliced_n = 0);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.
 uint32_t batched_tile_bound(const PlanTable& plan, uint32_t n);
 // Record a CUDA failure (message for myersGetErrorString) and return MYERS_E_CUDA.

@@ -85,10 +85,10 @@ struct SlicedClass {
 };
 
 // The classes; sliced_class (myers_internal.h) says which one a shape is in.
-using Sliced16 = SlicedClass<4, 4, 9, 16, false>;
+using Sliced16 = SlicedClass<4, 4, 8, 16, false>;
 using Sliced24 = SlicedClass<4, 3, 17, 24, false>;
 using Sliced32 = SlicedClass<4, 2, 25, 32, false>;
-using SlicedChain = SlicedClass<8, 1, 17, 40, true>;
+using SlicedChain = SlicedClass<8, 1, 8, 40, true>;
 
 // 3-input logic op by truth table (A 0xF0, B 0xCC, C 0xAA).
 constexpr int kA = 0xF0, kB = 0xCC, kC = 0xAA;

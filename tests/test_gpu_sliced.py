@@ -4,7 +4,8 @@ group, warps per group), lengths that differ within a group, groups that are
 not full, text and reads with N, PEQ rows with no base or with several, and
 the lengths a caller did not announce. Small batches take the word-parallel
 shapes, so each case runs in a child with MYERS_SLICED=1 (read once per
-process)."""
+process); 2 and 3 spread the shapes of reads of up to 512 bases over two and
+four times the lanes, as batches of many short lengths do."""
 import os
 import subprocess
 import sys
@@ -123,9 +124,13 @@ def run_unannounced():
     ctx.close()
 
 
-@pytest.mark.parametrize("name", [*CASES, "unannounced"])
-def test_sliced(name, cuda_ok):
+SPREAD = ["100b", "128b", "129b", "255b", "256b", "257b", "512b", "mixed", "ragged", "rows-without-base", "cutoff-ragged"]
+
+
+@pytest.mark.parametrize("name,mode", [*((n, "1") for n in [*CASES, "unannounced"]), *((n, "2") for n in SPREAD),
+                                       *((n, "3") for n in SPREAD)])
+def test_sliced(name, mode, cuda_ok):
     code = f"import test_gpu_sliced as t; t.run_unannounced() if {name!r} == 'unannounced' else t.run({name!r})"
     out = subprocess.run([sys.executable, "-c", code], cwd=os.path.join(ROOT, "tests"),
-                         env=dict(os.environ, MYERS_SLICED="1"), capture_output=True, text=True, timeout=600)
+                         env=dict(os.environ, MYERS_SLICED=mode), capture_output=True, text=True, timeout=600)
     assert out.returncode == 0, out.stderr[-2000:]
