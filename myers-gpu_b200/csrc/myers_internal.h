@@ -75,6 +75,10 @@ constexpr uint64_t kLargeBatchCandidates = 150000;
 // for reads of up to 1,024 bases: lanes of at most kSmallBatchLaneWords words.
 constexpr uint64_t kSmallBatchCandidates = 280000;
 constexpr uint32_t kSmallBatchLaneWords = 12;
+// Batches of fewer words per column than kFewWords, with reads of kFewMinWords
+// words or more among them, take lanes of at most kFewLaneWords words.
+constexpr uint64_t kFewWords = 400000;
+constexpr uint32_t kFewMinWords = 12, kFewLaneWords = 5;
 // With fewer than two candidates per read, reads of 513..1,024 bases take
 // lanes of at most this many words.
 constexpr uint32_t kDistinctLaneWords = 16;
