@@ -911,9 +911,10 @@ extern "C" int myersVerifyRangeAsync(myersContext_t* ctx, const myersReference_t
 // Ukkonen's cut-off (GEMTools/src/gt_map_align_bpm.c:141-210,
 // gt_map_block_bpm_get_distance__cutoff): the result is exact where the
 // minimum is at most (uint32_t)(m * cutoff), else {MYERS_NO_MATCH,
-// MYERS_NO_MATCH}. The plain path's single-lane shapes of 8..32 words (a
-// multiple of 4) skip the rows above the band; other shapes and the batched
-// path compute every row and apply the same contract.
+// MYERS_NO_MATCH}. The plain path's word-parallel single-lane shapes of 8..32
+// words (a multiple of 4) skip the rows above the band; the bit-sliced and the
+// other shapes and the batched path compute every row and apply the same
+// contract.
 extern "C" int myersVerifyCutoffAsync(myersContext_t* ctx, const myersReference_t* ref, const qryEntry_t* d_peq,
                                       uint32_t numPEQEntries, const qryInfo_t* d_qinfo, uint32_t numQueries,
                                       const candInfo_t* d_cands, uint32_t numCandidates, float distance,
@@ -1438,8 +1439,7 @@ extern "C" int myersReceive(void* mb) {
   CU(cudaStreamSynchronize(b->stream));
   if (b->pending) {
     b->pending = false;
-    if (*b->h_flags & kFlagTimeout) b->last_status = MYERS_E_TIMEOUT;
-    else if (*b->h_flags != 0) b->last_status = MYERS_E_QUERY_TOO_LONG;
+    if (*b->h_flags != 0) b->last_status = MYERS_E_QUERY_TOO_LONG;
   }
   return b->last_status;
 }

@@ -32,7 +32,6 @@ constexpr uint32_t kMaxColumns = 65535;       // the result key keeps 16 column 
 constexpr uint32_t kFlagUnsupported = 1u;     // query too long or window too wide
 constexpr uint32_t kFlagBadQuery = 2u;        // candidate query index >= numQueries
 constexpr uint32_t kFlagBadEntry = 4u;        // query PEQ entries beyond numPEQEntries
-constexpr uint32_t kFlagTimeout = 8u;         // a bounded wait inside a kernel gave up
 
 // Candidate as laid out by the API (candInfo_t with its 4 padding bytes).
 struct Cand {
