@@ -367,7 +367,9 @@ typedef struct {
  * (one pass's walk overlaps the next pass's recomputation), so half of it
  * must hold the band of the widest traced candidate, else myersTraceback
  * returns MYERS_E_CAPACITY: a read of 1000 bases needs about 90 KB at score
- * 60 and about 900 KB at score 600. Calls on one traceback object must be
+ * 60 and about 900 KB at score 600. (Bands of at most 15 words take one pass
+ * with a slot per resident warp where the scratch holds them; the capacity
+ * rule is the same.) Calls on one traceback object must be
  * ordered (one stream, or synchronised). */
 typedef struct myersTraceback myersTraceback_t;
 int myersTracebackCreate(myersTraceback_t **tb, uint64_t maxCandidates, uint64_t scratchBytes);

@@ -297,13 +297,16 @@ static bool small_batch(uint64_t n) {
 
 // Whether a batch is so small that the time of one tile counts, not the lanes'
 // efficiency: reads of up to 1,024 bases then take lanes of kFewLaneWords words
-// on either path (and in the serving loop, within its laneWords). The batch's
+// on either path. The batch's
 // words per column are estimated from the word counts that occur, 0.6 of the
 // middle where they differ. Measured on the batched path, against lanes of 12
 // words: 1,000 bases 110 candidates 0.21 -> 0.15 ms, 11K 0.46 -> 0.42, 22K 0.71 ->
 // 0.82; 400 bases 11K 0.151 -> 0.124, 33K 0.25 -> 0.27; 100..1,000 bases 1.1K 0.21 ->
 // 0.15, 11K 0.46 -> 0.29, 33K 0.46 -> 0.36, 66K 0.61 -> 0.63. On the plain path,
 // against one lane of 32 words: 1,000 bases 110 candidates 0.50 -> 0.14 ms.
+// Not in the serving loop, whose slots fill the device together: there 64
+// requests gained (733 -> 592 us), but 86M candidates/s offered had a p99 of
+// 3.6-8.4 ms instead of 1.6-2.3, and of 1.7-5.3 with a quarter of the threshold.
 static bool few_words(const uint8_t* present, uint64_t n) {
   if (!small_batch(n)) return false;
   uint32_t lo = 0, hi = 0;
@@ -427,7 +430,7 @@ static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words = 0, bool 
 // Build the plan for the word counts flagged in `present` (size kMaxWords+1).
 // Uses fixed-size stack arrays only: no allocation on the send path.
 int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, uint64_t n,
-                      uint64_t reads, Lengths lengths, bool bucketed, uint64_t sliced_n) {
+                      uint64_t reads, Lengths lengths, bool bucketed, uint64_t sliced_n, bool unshared) {
   memset(&t, 0, sizeof(t));
   memset(t.cfg_of_words, kNoCfg, sizeof(t.cfg_of_words));
   memset(t.cfg_of_sliced, kNoCfg, sizeof(t.cfg_of_sliced));
@@ -437,7 +440,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   int nshapes = 0;
   for (uint32_t w = 0; w <= kMaxWords; ++w) cfg_of[w] = -1;
   const bool small = batched && lane_words == 0 && small_batch(n);
-  const bool few = few_words(present, n);
+  const bool few = unshared && few_words(present, n);
   // Fewer than two candidates per read: a warp of 32 one-lane candidates then
   // holds more distinct reads than the 16 PEQ slots of the single-lane shapes
   // of more than 16 words, and runs its lanes in two rounds. Lanes of at most
@@ -481,7 +484,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     }
     alone = false;
     uint32_t lw = lane_words;
-    if (few && w <= 32) lw = lane_words > 0 && lane_words < kFewLaneWords ? lane_words : kFewLaneWords;
+    if (few && w <= 32) lw = kFewLaneWords;
     else if (small && w <= 32) lw = kSmallBatchLaneWords;
     else if (distinct && w > kDistinctLaneWords && w <= 32) lw = kDistinctLaneWords;
     const Shape s = pick_shape(w, batched, lw, large_batch(n));

@@ -296,11 +296,13 @@ cudaError_t launch_lop3_probe(uint32_t* d_out, int blocks, int threads, int iter
 // bucketed: the candidates will be classified by the plan in any case, so it
 // names every shape of the word counts present.
 // sliced_n: candidates expected, where they are not n (the cut-off's second pass).
+// unshared: no other batches share the device (a server's do).
 struct Lengths {
   uint32_t lo = 0, hi = 0;  // 0, 0: unknown
 };
 int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words = 0, uint64_t n = 0,
-               uint64_t reads = 0, Lengths lengths = {}, bool bucketed = false, uint64_t sliced_n = 0);
+               uint64_t reads = 0, Lengths lengths = {}, bool bucketed = false, uint64_t sliced_n = 0,
+               bool unshared = true);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.
 uint32_t batched_tile_bound(const PlanTable& plan, uint32_t n);
 // Record a CUDA failure (message for myersGetErrorString) and return MYERS_E_CUDA.
