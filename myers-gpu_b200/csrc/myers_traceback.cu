@@ -148,8 +148,8 @@ __device__ __forceinline__ uint32_t tb_setup(const TbArgs& a, uint32_t id, uint2
   g.m = q.y;
   g.pos_entry = q.x;
   g.s = res.y;
-  g.c1 = res.x + 1u;
-  if (g.c1 > n || n > kMaxColumns || g.m > kMaxWords * 32u) return kTbInconsistent;
+  if (res.x >= n || n > kMaxColumns || g.m > kMaxWords * 32u) return kTbInconsistent;
+  g.c1 = res.x + 1u;  // 1..n: column 0xFFFFFFFF must not wrap to 0
   if (g.m == 0) return (res.x == 0 && res.y == 0) ? 1u : kTbInconsistent;
   if (g.s > g.m) return kTbInconsistent;  // D[m][j] <= m for every column
   g.off = (int)g.c1 - (int)g.m;
