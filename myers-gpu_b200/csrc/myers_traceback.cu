@@ -1039,7 +1039,10 @@ static cudaError_t plan_tb_band(BandLaunch& l, uint32_t count, uint32_t band, ui
   const uint32_t window = WMAX > 7 && band < 9u ? 9u : band <= 3u ? 3u : band | 1u;
   l.warp_words = window * (BandMem<WMAX>::kWords / WMAX);
   l.smem = (size_t)kBandWarps * l.warp_words * 4;
-  cudaError_t e = cudaFuncSetAttribute(k_tb_band<WMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
+  // The limit belongs to the function, not to the launch: always that of the
+  // widest window, so that calls on other threads can't lower it in between.
+  cudaError_t e = cudaFuncSetAttribute(k_tb_band<WMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kBandWarps * BandMem<WMAX>::kWords * 4u));
   int per_sm = 0;
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tb_band<WMAX>, 32 * kBandWarps, l.smem);
   if (e != cudaSuccess) return e;
@@ -1051,6 +1054,17 @@ static cudaError_t plan_tb_band(BandLaunch& l, uint32_t count, uint32_t band, ui
   l.blocks = (uint32_t)blocks;
   return cudaSuccess;
 }
+
+// While it is open, a call that returns early waits for what it put on the
+// walk's stream: the caller's stream would not, and the next call clears the
+// state under it.
+struct WalkGuard {
+  cudaStream_t walk;
+  bool open = true;
+  ~WalkGuard() {
+    if (open) cudaStreamSynchronize(walk);
+  }
+};
 
 // Trace the whole list with the banded kernel: in bucket order, bands of more
 // than 7 words on the walk's stream beside the others. False in `done` where a
@@ -1169,11 +1183,13 @@ extern "C" int myersTraceback(myersTraceback_t* tb, const myersReference_t* ref,
   // the last of them ends within H + max_units <= half the scratch
   const unsigned long long half_units = (tb->scratch_bytes / 2) >> kTbUnitShift;
   if (half_units <= st.max_units) return MYERS_E_CAPACITY;  // one band does not fit half the scratch
+  WalkGuard guard{tb->walk_stream};
   {
     bool done = false;
     const int bs = trace_bands(tb, a, st, s, done);
     if (bs != MYERS_SUCCESS) return bs;
     if (done) {
+      guard.open = false;
       tb->last_chunks = 1;
       return MYERS_SUCCESS;
     }
@@ -1210,5 +1226,6 @@ extern "C" int myersTraceback(myersTraceback_t* tb, const myersReference_t* ref,
   tb->last_chunks = c;
   // the caller's stream resumes after the last walk
   if ((e = cudaStreamWaitEvent(s, tb->walk_done[(c - 1u) & 1u], 0)) != cudaSuccess) return cuda_fail(e, "wait");
+  guard.open = false;
   return MYERS_SUCCESS;
 }
