@@ -449,16 +449,11 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   // Bit-sliced shapes: for the word counts without an override, every length
   // of a word count that is present (lengths the caller did not announce but
   // whose word count occurs are admitted, as by the word-parallel shapes).
-  const bool sliced = lane_words == 0 && (!few || sliced_force() > 0) && sliced_batch(lengths, batched, sliced_n ? sliced_n : n, t.spread);
+  bool sliced = lane_words == 0 && (!few || sliced_force() > 0) && sliced_batch(lengths, batched, sliced_n ? sliced_n : n, t.spread);
   uint8_t sliced_words[kMaxWords + 1];
   memset(sliced_words, 0, sizeof(sliced_words));
   uint32_t sliced_rows[kSlicedShapes];  // longest length of each bit-sliced shape
   memset(sliced_rows, 0, sizeof(sliced_rows));
-  if (sliced) {
-    std::lock_guard<std::mutex> lk(g_override_mu);
-    for (uint32_t w = kSlicedMinRows / 32 + 1; w <= kSlicedMaxRows / 32; ++w)
-      sliced_words[w] = present[w] && !g_override[batched ? 1 : 0][w].set;
-  }
   // every length that can occur has the same bit-sliced shape (a longer length
   // never has a smaller one)
   bool alone = sliced && !bucketed && lengths.lo >= kSlicedMinRows && lengths.hi <= kSlicedMaxRows;
@@ -467,12 +462,29 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     int lg, R;
     alone_shape = sliced_shape(lengths.lo, t.spread, &lg, &R);
     alone = alone_shape == sliced_shape(lengths.hi, t.spread, &lg, &R);
+    // One shape for every candidate, so no bucketing: admit the lengths the
+    // word-parallel shape would (all that fit its rows on the plain path, the
+    // word counts present on the batched path), as far as a bit-sliced tile can
+    // fall back to the word-parallel one.
+    const uint32_t w_lo = (lengths.lo + 31) / 32, w_hi = (lengths.hi + 31) / 32;
+    t.row_min = 1;
+    t.row_limit = 32 * w_hi;
+    if (batched) {
+      t.row_min = 32 * (w_lo - 1) + 1;
+    } else {
+      const Shape s = pick_shape(w_hi, batched, distinct && w_hi > kDistinctLaneWords && w_hi <= 32 ? kDistinctLaneWords : 0,
+                                 large_batch(n));
+      t.row_limit = 32u * s.W * s.L;
+    }
+    if (t.row_limit > (lg > 5 ? kSlicedChainWordRows : kSlicedWordRows)) sliced = alone = false;
   }
-  uint32_t w_lo = 0, w_hi = 0;
+  if (sliced) {
+    std::lock_guard<std::mutex> lk(g_override_mu);
+    for (uint32_t w = kSlicedMinRows / 32 + 1; w <= kSlicedMaxRows / 32; ++w)
+      sliced_words[w] = present[w] && !g_override[batched ? 1 : 0][w].set;
+  }
   for (uint32_t w = 1; w <= kMaxWords; ++w) {
     if (!present[w]) continue;
-    if (w_lo == 0) w_lo = w;
-    w_hi = w;
     if (sliced_words[w]) {
       t.cfg_of_words[w] = kSlicedCfg;
       for (uint32_t m = 32 * (w - 1) + 1; m <= 32 * w; ++m) {
@@ -510,20 +522,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     max_words[nshapes] = sliced_rows[i];
     ++nshapes;
   }
-  if (alone) {
-    // One shape for every candidate, so no bucketing: admit the lengths the
-    // word-parallel shape would (all that fit its rows on the plain path, the
-    // word counts present on the batched path).
-    t.row_min = 1;
-    t.row_limit = 32 * w_hi;
-    if (batched) {
-      t.row_min = 32 * (w_lo - 1) + 1;
-    } else {
-      const Shape s = pick_shape(w_hi, batched, distinct && w_hi > kDistinctLaneWords && w_hi <= 32 ? kDistinctLaneWords : 0,
-                                 large_batch(n));
-      t.row_limit = 32u * s.W * s.L;
-    }
-  }
+  if (!alone) t.row_min = t.row_limit = 0;
   // order: persistent-kernel shapes first, then bit-sliced ones, then the rest,
   // each group by decreasing cost
   int order[kMaxCfg];
@@ -877,8 +876,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
   return MYERS_SUCCESS;
 }
 
-static int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n,
-                          uint64_t reads) {
+int myers::plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads) {
   uint8_t present[kMaxWords + 1];
   memset(present, 0, sizeof(present));
   if (maxSize == 0) maxSize = kMaxWords * 32;

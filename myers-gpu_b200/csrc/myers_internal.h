@@ -95,6 +95,9 @@ constexpr uint8_t kSlicedVariant = 0xFE;
 constexpr uint8_t kSlicedCfg = 0xFE;    // cfg_of_words: look in cfg_of_sliced
 constexpr uint32_t kSlicedMinRows = 65, kSlicedMaxRows = 10240;
 constexpr int kSlicedMinLg = 3, kSlicedMaxLg = 8, kSlicedMinR = 8, kSlicedMaxR = 40;
+// Rows of the word-parallel tile that a bit-sliced tile falls back to: 32 lanes
+// of 4 words, of 16 in groups of several warps.
+constexpr uint32_t kSlicedWordRows = 4096, kSlicedChainWordRows = 16384;
 constexpr int kSlicedShapes = (kSlicedMaxLg - kSlicedMinLg + 1) * (kSlicedMaxR - kSlicedMinR + 1);
 
 // Index of the bit-sliced shape of m rows (kSlicedMinRows..kSlicedMaxRows).
@@ -303,6 +306,8 @@ struct Lengths {
 int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words = 0, uint64_t n = 0,
                uint64_t reads = 0, Lengths lengths = {}, bool bucketed = false, uint64_t sliced_n = 0,
                bool unshared = true);
+// The plan of a call whose queries have minSize..maxSize bases (0, 0: any).
+int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.
 uint32_t batched_tile_bound(const PlanTable& plan, uint32_t n);
 // Record a CUDA failure (message for myersGetErrorString) and return MYERS_E_CUDA.

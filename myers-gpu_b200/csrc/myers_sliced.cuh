@@ -651,7 +651,8 @@ __global__ void __launch_bounds__(K::kThreads, K::kBlocks)
     t.R = s.W;
     t.lg = s.L;
     t.row_min = plan.row_min;
-    t.row_limit = plan.row_limit ? plan.row_limit : (uint32_t)s.W << s.L;
+    t.row_limit = min(plan.row_limit ? plan.row_limit : (uint32_t)s.W << s.L,
+                      K::kChain ? kSlicedChainWordRows : kSlicedWordRows);  // run_words' tile
     t.nw = K::kChain ? 1 << (s.L - 5) : 1;
     t.wg = warp & (t.nw - 1);
     t.group = warp / t.nw;

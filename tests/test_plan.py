@@ -1,0 +1,41 @@
+"""The choice of kernel shapes, on the CPU: plan_dump.cpp prints the plan that a
+call would take and the query lengths that it admits."""
+import json
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "myers-gpu_b200")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+PLAIN, BATCHED = 0, 1
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("plan") / "plan_dump")
+    subprocess.run(["g++", "-O1", "-std=c++17", f"-I{CUDA}/include", f"-I{PKG}/csrc", "-o", exe,
+                    os.path.join(ROOT, "tests", "plan_dump.cpp"), os.path.join(PKG, "libmyers_b200.so"),
+                    f"-Wl,-rpath,{PKG}"], check=True)
+
+    def dump(path, lo, hi, n, reads=0, cut=-1.0, **env):
+        env = {k: v for k, v in os.environ.items() if not k.startswith("MYERS_")} | env
+        out = subprocess.run([exe, str(path), str(lo), str(hi), str(n), str(reads), str(cut)], env=env, check=True,
+                             capture_output=True, text=True)
+        return json.loads(out.stdout)
+    return dump
+
+
+@pytest.mark.parametrize("words,shape,length", [(32, [32, 8], 1000), (32, [32, 32], 1000), (16, [16, 32], 500),
+                                                (40, [32, 32], 1270), (300, [32, 32], 9590)])
+def test_bit_sliced_tiles_can_fall_back(plan, tmp_path, words, shape, length):
+    """A lone bit-sliced shape admits the lengths of the word-parallel shape that
+    it replaces. Its tiles fall back to word-parallel ones of 4,096 rows (16,384 in
+    groups of several warps), so a tuned shape of more rows keeps its place."""
+    fn = tmp_path / "tuned.json"
+    fn.write_text(json.dumps({"plain": {str(words): shape}, "batched": {}, "batched_large": {}}))
+    p = plan(PLAIN, length, length, 2_000_000, 100_000, MYERS_AUTOTUNE=str(fn))["plan"]
+    if p["sliced"]:
+        assert p["admits"][-1][1] <= (4096 if length <= 1024 else 16384)
+    assert p["admits"] == [[1, 32 * shape[0] * shape[1]]]
