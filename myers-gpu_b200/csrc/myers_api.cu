@@ -371,6 +371,9 @@ static bool sliced_batch(Lengths len, bool batched, uint64_t n, uint32_t& spread
   return rounds >= 4 || 10 * tiles >= 7 * rounds * round;
 }
 
+// Fewer than two candidates per read (0 reads: unknown).
+static bool few_candidates(uint64_t n, uint64_t reads) { return reads > 0 && n < 2 * reads; }
+
 // lane_words > 0 asks for latency-oriented shapes: a query of more than
 // lane_words words is spread over ceil(words / W) lanes of W <= lane_words
 // words, the cheapest such shape by the cost model (shorter per-candidate
@@ -427,10 +430,32 @@ static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words = 0, bool 
   return bs;
 }
 
+// Whether the word-parallel shapes of the word counts present are one shape on
+// the plain path, and its rows.
+static bool one_plain_shape(const uint8_t* present, uint64_t n, uint64_t reads, uint32_t& rows) {
+  bool any = false;
+  Shape one{0, 0, 0, 0};
+  for (uint32_t w = 1; w <= kMaxWords; ++w) {
+    if (!present[w]) continue;
+    const Shape s = pick_shape(w, false, few_candidates(n, reads) && w > kDistinctLaneWords && w <= 32 ? kDistinctLaneWords : 0,
+                               large_batch(n));
+    if (any && (s.variant != one.variant || s.L != one.L)) return false;
+    one = s;
+    any = true;
+  }
+  rows = 32u * one.W * one.L;
+  return any;
+}
+
 // Build the plan for the word counts flagged in `present` (size kMaxWords+1).
 // Uses fixed-size stack arrays only: no allocation on the send path.
-int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, uint64_t n,
-                      uint64_t reads, Lengths lengths, bool bucketed, uint64_t sliced_n, bool unshared) {
+//
+// Which lengths it admits doesn't depend on the shapes it takes. On the batched
+// path they are those of the word counts present. On the plain path, where the
+// word-parallel shapes of these word counts are one, every length that fits
+// this shape's rows is admitted, as a launch without bucketing admits it; else
+// again those of the word counts present.
+int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, const Batch& b) {
   memset(&t, 0, sizeof(t));
   memset(t.cfg_of_words, kNoCfg, sizeof(t.cfg_of_words));
   memset(t.cfg_of_sliced, kNoCfg, sizeof(t.cfg_of_sliced));
@@ -439,44 +464,50 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   int16_t cfg_of[kMaxWords + 1];
   int nshapes = 0;
   for (uint32_t w = 0; w <= kMaxWords; ++w) cfg_of[w] = -1;
+  const uint64_t n = b.n;
+  const Lengths lengths = b.lengths;
+  t.bucketed = b.bucketed;
+  uint32_t w_lo = 0, w_hi = 0;
+  for (uint32_t w = 1; w <= kMaxWords; ++w)
+    if (present[w]) {
+      if (w_lo == 0) w_lo = w;
+      w_hi = w;
+    }
+  if (w_lo == 0) return MYERS_SUCCESS;
   const bool small = batched && lane_words == 0 && small_batch(n);
-  const bool few = unshared && few_words(present, n);
+  const bool few = b.unshared && few_words(present, n);
   // Fewer than two candidates per read: a warp of 32 one-lane candidates then
   // holds more distinct reads than the 16 PEQ slots of the single-lane shapes
   // of more than 16 words, and runs its lanes in two rounds. Lanes of at most
   // 16 words stage each lane's own words instead.
-  const bool distinct = lane_words == 0 && reads > 0 && n < 2 * reads;
+  const bool distinct = lane_words == 0 && few_candidates(n, b.reads);
   // Bit-sliced shapes: for the word counts without an override, every length
   // of a word count that is present (lengths the caller did not announce but
   // whose word count occurs are admitted, as by the word-parallel shapes).
-  bool sliced = lane_words == 0 && (!few || sliced_force() > 0) && sliced_batch(lengths, batched, sliced_n ? sliced_n : n, t.spread);
+  bool sliced = lane_words == 0 && (!few || sliced_force() > 0) &&
+                sliced_batch(lengths, batched, b.sliced_n ? b.sliced_n : n, t.spread);
+  // the rows admitted
+  const bool adapts = few || sliced;
+  uint32_t row_min = 32 * (w_lo - 1) + 1, row_limit = 32 * w_hi, one_rows = 0;
+  const bool by_rows = (adapts || b.bucketed) && !batched && !b.by_words && one_plain_shape(present, n, b.reads, one_rows);
+  if (by_rows) {
+    row_min = 1;
+    row_limit = one_rows;
+  }
+  // as far as a bit-sliced tile can fall back to the word-parallel one
+  if (sliced && row_limit > (lengths.hi > 1024 ? kSlicedChainWordRows : kSlicedWordRows) && by_rows) sliced = false;
   uint8_t sliced_words[kMaxWords + 1];
   memset(sliced_words, 0, sizeof(sliced_words));
   uint32_t sliced_rows[kSlicedShapes];  // longest length of each bit-sliced shape
   memset(sliced_rows, 0, sizeof(sliced_rows));
   // every length that can occur has the same bit-sliced shape (a longer length
-  // never has a smaller one)
-  bool alone = sliced && !bucketed && lengths.lo >= kSlicedMinRows && lengths.hi <= kSlicedMaxRows;
+  // never has a smaller one): one shape for every candidate, so no bucketing
+  bool alone = sliced && !b.bucketed && lengths.lo >= kSlicedMinRows && lengths.hi <= kSlicedMaxRows;
   int alone_shape = -1;
   if (alone) {
     int lg, R;
     alone_shape = sliced_shape(lengths.lo, t.spread, &lg, &R);
     alone = alone_shape == sliced_shape(lengths.hi, t.spread, &lg, &R);
-    // One shape for every candidate, so no bucketing: admit the lengths the
-    // word-parallel shape would (all that fit its rows on the plain path, the
-    // word counts present on the batched path), as far as a bit-sliced tile can
-    // fall back to the word-parallel one.
-    const uint32_t w_lo = (lengths.lo + 31) / 32, w_hi = (lengths.hi + 31) / 32;
-    t.row_min = 1;
-    t.row_limit = 32 * w_hi;
-    if (batched) {
-      t.row_min = 32 * (w_lo - 1) + 1;
-    } else {
-      const Shape s = pick_shape(w_hi, batched, distinct && w_hi > kDistinctLaneWords && w_hi <= 32 ? kDistinctLaneWords : 0,
-                                 large_batch(n));
-      t.row_limit = 32u * s.W * s.L;
-    }
-    if (t.row_limit > (lg > 5 ? kSlicedChainWordRows : kSlicedWordRows)) sliced = alone = false;
   }
   if (sliced) {
     std::lock_guard<std::mutex> lk(g_override_mu);
@@ -499,7 +530,8 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     if (few && w <= 32) lw = kFewLaneWords;
     else if (small && w <= 32) lw = kSmallBatchLaneWords;
     else if (distinct && w > kDistinctLaneWords && w <= 32) lw = kDistinctLaneWords;
-    const Shape s = pick_shape(w, batched, lw, large_batch(n));
+    Shape s = pick_shape(w, batched, lw, large_batch(n));
+    if (by_rows && 32u * s.W * s.L < row_limit) s = pick_shape(row_limit / 32, batched, lw, large_batch(n));
     if (s.L == 0) return MYERS_E_QUERY_TOO_LONG;
     int found = -1;
     for (int i = 0; i < nshapes; ++i)
@@ -522,7 +554,10 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     max_words[nshapes] = sliced_rows[i];
     ++nshapes;
   }
-  if (!alone) t.row_min = t.row_limit = 0;
+  if (by_rows || (adapts && !b.bucketed && nshapes == 1)) {
+    t.row_min = row_min;
+    t.row_limit = row_limit;
+  }
   // order: persistent-kernel shapes first, then bit-sliced ones, then the rest,
   // each group by decreasing cost
   int order[kMaxCfg];
@@ -562,6 +597,13 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   }
   for (uint32_t w = 1; w <= kMaxWords; ++w)
     if (cfg_of[w] >= 0) t.cfg_of_words[w] = (uint8_t)rank[cfg_of[w]];
+  if (by_rows && (b.bucketed || nshapes > 1)) {
+    // Shorter lengths than those present fit the first one's shape; longer ones go
+    // to the last one's, which verifies them up to row_limit and flags the rest.
+    const uint8_t first = (uint8_t)plan_cfg(t, 32 * (w_lo - 1) + 1), last = (uint8_t)plan_cfg(t, 32 * w_hi);
+    for (uint32_t w = 1; w <= kMaxWords; ++w)
+      if (!present[w]) t.cfg_of_words[w] = w < w_lo ? first : last;
+  }
   return MYERS_SUCCESS;
 }
 
@@ -687,13 +729,25 @@ int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* presen
     }
   }
   // the second pass holds the candidates that survived, mostly one per read
+  uint32_t rows = 0;
+  bool any2 = false;
+  for (uint32_t w = 1; w <= kMaxWords && !any2; ++w) any2 = w2[w];
+  const bool by_words = batched || !one_plain_shape(w1, n, 0, rows) || (any2 && !one_plain_shape(w2, n, n, rows));
   auto both = [&](bool bucketed) {
-    const int st = build_plan(plan, w1, batched, 0, n, 0, m1, bucketed);
-    return st != MYERS_SUCCESS ? st : build_plan(plan2, w2, batched, 0, n, n, m2, bucketed, n / 8);
+    Batch b;
+    b.n = n;
+    b.lengths = m1;
+    b.bucketed = bucketed;
+    b.by_words = by_words;
+    const int st = build_plan(plan, w1, batched, 0, b);
+    b.reads = n;
+    b.lengths = m2;
+    b.sliced_n = n / 8;
+    return st != MYERS_SUCCESS ? st : build_plan(plan2, w2, batched, 0, b);
   };
-  int st = both(batched);
+  int st = both(by_words);
   // more than one shape in either pass: both are classified
-  if (st == MYERS_SUCCESS && !batched && (plan.num_cfg > 1 || plan2.num_cfg > 1)) st = both(true);
+  if (st == MYERS_SUCCESS && !by_words && (plan.num_cfg > 1 || plan2.num_cfg > 1)) st = both(true);
   return st;
 }
 
@@ -722,6 +776,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
   in.ref_words = ref->words + kRefPadWords;
   in.flags = ctx->d_flags;
   set_multipliers(in);
+  admit(in, plan);
   ctx->last_launches = 0;
   if (in.num_cands == 0) return MYERS_SUCCESS;
   if (in.num_cands > ctx->capacity) return MYERS_E_CAPACITY;
@@ -800,6 +855,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
     CU(shapes_enqueue(plan, in, ctx->d_ids, ctx->d_state, plan.num_batched, &launches));
     DevInputs in2 = in;
     in2.prefix = 0;
+    admit(in2, *plan2);
     CU(launch_plan_tiles(*plan2, ctx->d_esc_state, s));
     ++launches;
     if (plan2->num_batched > 0) {
@@ -823,7 +879,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
     in.esc_state = ctx->d_esc_state;
     CU(cudaMemsetAsync(ctx->d_esc_state, 0, sizeof(BucketState), s));
     uint32_t launches = 0;
-    if (plan.num_cfg <= 1 && plan2->num_cfg <= 1) {
+    if (!plan.bucketed) {
       in.esc_cfg = nullptr;  // one full-length shape: list 0
       if (plan.num_cfg == 1) {
         uint32_t* next = &ctx->d_state->next[0];
@@ -843,6 +899,7 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
     }
     DevInputs in2 = in;
     in2.prefix = 0;
+    admit(in2, *plan2);
     CU(shapes_enqueue(*plan2, in2, ctx->d_esc_ids, ctx->d_esc_state, 0, &launches));
     ctx->last_launches = launches;
     return MYERS_SUCCESS;
@@ -883,7 +940,11 @@ int myers::plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, i
   if (maxSize > kMaxWords * 32) maxSize = kMaxWords * 32;
   const uint32_t wlo = minSize ? (minSize + 31) / 32 : 1, whi = (maxSize + 31) / 32;
   for (uint32_t w = wlo; w <= whi; ++w) present[w] = 1;
-  return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, n, reads, Lengths{minSize ? minSize : 1, maxSize});
+  Batch b;
+  b.n = n;
+  b.reads = reads;
+  b.lengths = Lengths{minSize ? minSize : 1, maxSize};
+  return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, b);
 }
 
 extern "C" int myersVerifyAsync(myersContext_t* ctx, const myersReference_t* ref, const qryEntry_t* d_peq,
@@ -1357,8 +1418,11 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
       st = cutoff_plans(plan, b->plan2, pm.data(), b->cutoff, cutoff_prefix_mult(), b->path == MYERS_PATH_BATCHED,
                         numCandidates);
     } else {
-      st = build_plan(plan, present.data(), b->path == MYERS_PATH_BATCHED, 0, numCandidates / parts,
-                      numQueries / parts, lengths);
+      Batch batch;
+      batch.n = numCandidates / parts;
+      batch.reads = numQueries / parts;
+      batch.lengths = lengths;
+      st = build_plan(plan, present.data(), b->path == MYERS_PATH_BATCHED, 0, batch);
     }
   }
   if (st != MYERS_SUCCESS) return b->last_status = st;
@@ -1629,6 +1693,7 @@ extern "C" int myersVerifyNoAllocAsync(const uint32_t* d_refWords, uint64_t refW
   in.distance = distance;
   in.exact = windowMode == MYERS_WINDOW_EXACT;
   set_multipliers(in);
+  admit(in, plan);
   cudaStream_t s = (cudaStream_t)stream;
   // the array keeps the previous call's contents: the bucket table (counts,
   // cursors, work queue) and the flags must start at zero

@@ -124,7 +124,8 @@ struct PlanTable {
   uint32_t num_batched;
   uint32_t num_sliced;
   uint32_t spread;     // of the bit-sliced shapes
-  uint32_t row_min, row_limit;  // one bit-sliced shape without bucketing: the queries it admits (else 0, 0)
+  uint32_t bucketed;   // the candidates are to be classified, also where there is one shape
+  uint32_t row_min, row_limit;  // the rows admitted (0, 0: what the shapes hold)
   Shape shape[kMaxCfg];
 };
 
@@ -181,6 +182,7 @@ struct DevInputs {
   // Multipliers the compiler cannot fold (set by set_multipliers): they keep
   // the per-column bookkeeping on the FMA pipe (see myers_kernels.cu).
   uint32_t one, two, k16, mk16, p28, kb33, kb17, mn16, mone;
+  uint32_t row_min, row_limit;   // rows admitted, besides what a shape holds (set by admit)
 };
 
 inline void set_multipliers(DevInputs& in) {
@@ -193,6 +195,12 @@ inline void set_multipliers(DevInputs& in) {
   in.kb17 = 17u * 4u * 4u;  // ... 17 columns
   in.mn16 = 0xFFFFFFF0u;    // -16
   in.mone = 0xFFFFFFFFu;    // -1
+}
+
+// The rows that the plan admits, for the launches over its shapes.
+inline void admit(DevInputs& in, const PlanTable& plan) {
+  in.row_min = plan.row_limit ? plan.row_min : 0u;
+  in.row_limit = plan.row_limit ? plan.row_limit : 0xFFFFFFFFu;
 }
 
 inline int variant_W(int v) { return v < kNumSingle ? v + 1 : kMultiW[v - kNumSingle]; }
@@ -291,21 +299,20 @@ cudaError_t launch_lop3_probe(uint32_t* d_out, int blocks, int threads, int iter
 // ---- host runtime internals (myers_api.cu) ----
 
 // Shape plan for the word counts flagged in present[0..kMaxWords].
-// n: the batch's candidates, which picks the batched path's table for large
-// batches at kLargeBatchCandidates or more.
-// reads: how many reads the n candidates come from (0: unknown).
-// lengths: the shortest and longest query that can occur; with them, large
-// batches take bit-sliced shapes.
-// bucketed: the candidates will be classified by the plan in any case, so it
-// names every shape of the word counts present.
-// sliced_n: candidates expected, where they are not n (the cut-off's second pass).
-// unshared: no other batches share the device (a server's do).
 struct Lengths {
   uint32_t lo = 0, hi = 0;  // 0, 0: unknown
 };
-int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words = 0, uint64_t n = 0,
-               uint64_t reads = 0, Lengths lengths = {}, bool bucketed = false, uint64_t sliced_n = 0,
-               bool unshared = true);
+struct Batch {
+  uint64_t n = 0;         // candidates
+  uint64_t reads = 0;     // reads they come from (0: unknown)
+  Lengths lengths;        // the shortest and longest query that can occur; with them, large batches take
+                          // bit-sliced shapes
+  uint64_t sliced_n = 0;  // candidates expected, where they are not n (the cut-off's second pass)
+  bool bucketed = false;  // the candidates will be classified in any case: name every shape of the word counts present
+  bool by_words = false;  // admit queries by their word counts alone
+  bool unshared = true;   // no other batches share the device (a server's do)
+};
+int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, const Batch& b);
 // The plan of a call whose queries have minSize..maxSize bases (0, 0: any).
 int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.

@@ -151,8 +151,11 @@ static int dispatch_slot(myersServer* srv, Slot& s) {
   }
   s.ncands = nc;
   PlanTable plan;
-  int st = build_plan(plan, present, srv->cfg.path == MYERS_PATH_BATCHED, srv->cfg.laneWords, nc, nq, Lengths{}, false, 0,
-                      /*unshared=*/false);
+  Batch batch;
+  batch.n = nc;
+  batch.reads = nq;
+  batch.unshared = false;
+  int st = build_plan(plan, present, srv->cfg.path == MYERS_PATH_BATCHED, srv->cfg.laneWords, batch);
   if (st != MYERS_SUCCESS) return st;
   // With graphs, the batch's copies and kernels are captured and replayed as
   // one graph, updated in place from the slot's previous batch.

@@ -427,7 +427,7 @@ __device__ __forceinline__ CandSetup setup_candidate(const DevInputs& in, const 
     const uint32_t wb = d_window_bases(c.mf, in.distance);
     const bool valid = bad == 0u && c.pos < in.ref_size && (in.ref_size - c.pos) > (unsigned long long)wb;
     c.n = in.exact ? wb : 8u * d_window_words(wb);
-    const bool fits = c.m <= (uint32_t)rows && c.n <= kMaxColumns;
+    const bool fits = c.m >= in.row_min && c.m <= min((uint32_t)rows, in.row_limit) && c.n <= kMaxColumns;
     c.qok = bad == 0u && c.m > 0 && c.m <= (uint32_t)rows;
     c.work = valid && c.m > 0 && fits;
     if (!c.work && l == 0) {

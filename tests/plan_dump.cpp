@@ -55,7 +55,7 @@ int main(int argc, char** argv) {
     std::vector<uint8_t> present(kMaxWords * 32 + 1, 0);
     for (uint32_t m = first; m <= last; ++m) present[m] = 1;
     if (cutoff_plans(a, b, present.data(), cut, cutoff_prefix_mult(), batched, n) != 0) return 1;
-    const bool unbucketed = !batched && a.num_cfg <= 1 && b.num_cfg <= 1;
+    const bool unbucketed = !batched && !a.bucketed;
     printf("{");
     print("first", a, unbucketed);
     printf(", ");

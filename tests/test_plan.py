@@ -1,7 +1,9 @@
 """The choice of kernel shapes, on the CPU: plan_dump.cpp prints the plan that a
 call would take and the query lengths that it admits."""
+import itertools
 import json
 import os
+import random
 import subprocess
 
 import pytest
@@ -39,3 +41,21 @@ def test_bit_sliced_tiles_can_fall_back(plan, tmp_path, words, shape, length):
     if p["sliced"]:
         assert p["admits"][-1][1] <= (4096 if length <= 1024 else 16384)
     assert p["admits"] == [[1, 32 * shape[0] * shape[1]]]
+
+
+RANGES = [(1, 32), (35, 301), (65, 96), (100, 100), (100, 128), (20, 1000), (545, 576), (640, 640), (700, 736), (900, 1000),
+          (930, 960), (940, 950), (961, 1000), (990, 1000), (1000, 1000), (1000, 1100), (1025, 1088), (1040, 1060),
+          (1500, 1600), (1505, 1568), (2000, 2048), (5000, 5100), (9000, 9600), (10000, 10200), (1000, 12000), (0, 0)]
+CALLS = list(itertools.product((PLAIN, BATCHED), RANGES, (100, 3000, 20_000, 120_000, 1_000_000), (1, 11),
+                               (-1.0, 0.0, 0.04, 0.2, 1.0)))
+
+
+@pytest.mark.parametrize("mode", ["", "1", "2", "3"])
+def test_admitted_lengths_do_not_depend_on_the_shapes(plan, mode):
+    """The lengths that a call verifies, those its range leaves out among them, are
+    the same whether it takes bit-sliced shapes, lanes of few words or neither."""
+    for path, (lo, hi), n, per_read, cut in random.Random(mode).sample(CALLS, 250):
+        got = plan(path, lo, hi, n, n // per_read, cut, **({"MYERS_SLICED": mode} if mode else {}))
+        expect = plan(path, lo, hi, n, n // per_read, cut, MYERS_SLICED="0", MYERS_SMALL_BATCH="0")
+        for part in expect:
+            assert got[part]["admits"] == expect[part]["admits"], (path, lo, hi, n, per_read, cut, part)
