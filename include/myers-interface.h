@@ -474,18 +474,21 @@ int myersNumVariants(void);
 int myersVariantWords(int variant);
 int myersVariantIsMulti(int variant);
 
-/* Shape the given path uses for a query length. */
+/* Word-parallel shape of a query length on the given path, of batches that take
+ * word-parallel shapes and no latency shapes. */
 int myersShapeOf(int path, uint32_t querySize, int *variant, int *L, int *W);
 
 /* Force the shape used for queries of `words` 32-bit words
  * (ceil(size/32)); variant -1 restores the built-in choice. */
 int myersSetShapeOverride(int path, uint32_t words, int variant, int L);
 
-/* Shapes come, in this order, from myersSetShapeOverride, the serving loop's
- * latency policy (laneWords), the autotuner's cache -- autotune_b200.json next
- * to the library, written by myers-gpu_b200/autotune.py (MYERS_AUTOTUNE names
- * another file, MYERS_AUTOTUNE=0 ignores it) -- and a built-in cost model.
- * Returns how many word counts the loaded cache covers for the path. */
+/* Shapes come, in this order, from myersSetShapeOverride, the latency policies
+ * (the serving loop's laneWords; small batches on the batched path), an
+ * autotuner's cache that MYERS_AUTOTUNE names, the rules that give large batches
+ * bit-sliced shapes and the smallest ones lanes of few words, the autotuner's
+ * cache next to the library -- autotune_b200.json, written by
+ * myers-gpu_b200/autotune.py (MYERS_AUTOTUNE=0 ignores it) -- and a built-in cost
+ * model. Returns how many word counts the loaded cache covers for the path. */
 int myersTunedShapes(int path);
 
 /* Integer-ALU throughput probe on the current device: 3-input logic ops per

@@ -192,6 +192,9 @@ static Override g_override[2][kMaxWords + 1];
 // from the autotuner's cache file: plain, batched, and batched for large
 // batches (see large_batch)
 static Override g_tuned[3][kMaxWords + 1];
+// whether MYERS_AUTOTUNE named that file: its shapes then stand as they are, while
+// those of the file beside the library are the best of the word-parallel ones
+static bool g_tuned_named = false;
 
 // Load the autotuner's cache: `autotune_b200.json` next to this library (or
 // the file named by MYERS_AUTOTUNE; MYERS_AUTOTUNE=0 disables it). Format:
@@ -221,6 +224,7 @@ static void load_tuned_once() {
     while ((n = fread(buf, 1, sizeof(buf), fp)) > 0) text.append(buf, n);
     fclose(fp);
     std::lock_guard<std::mutex> lk(g_override_mu);
+    g_tuned_named = env && *env;
     for (int path_id = 0; path_id < 3; ++path_id) {
       const char* key = path_id == 0 ? "\"plain\"" : path_id == 1 ? "\"batched\"" : "\"batched_large\"";
       size_t at = text.find(key);
@@ -266,6 +270,12 @@ static bool large_batch(uint64_t n) {
     return env ? strtoull(env, nullptr, 10) : (uint64_t)kLargeBatchCandidates;
   }();
   return n >= threshold;
+}
+
+// Whether a file that MYERS_AUTOTUNE names has a shape for w words (call with
+// g_override_mu held).
+static bool tuned_by_name(uint32_t w, bool batched, uint64_t n) {
+  return g_tuned_named && (g_tuned[batched ? 1 : 0][w].set || (batched && large_batch(n) && g_tuned[2][w].set));
 }
 
 // How many of a context's streams the plain path spreads its launches over
@@ -456,6 +466,7 @@ static bool one_plain_shape(const uint8_t* present, uint64_t n, uint64_t reads, 
 // this shape's rows is admitted, as a launch without bucketing admits it; else
 // again those of the word counts present.
 int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, const Batch& b) {
+  load_tuned_once();
   memset(&t, 0, sizeof(t));
   memset(t.cfg_of_words, kNoCfg, sizeof(t.cfg_of_words));
   memset(t.cfg_of_sliced, kNoCfg, sizeof(t.cfg_of_sliced));
@@ -496,6 +507,11 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   }
   // as far as a bit-sliced tile can fall back to the word-parallel one
   if (sliced && row_limit > (lengths.hi > 1024 ? kSlicedChainWordRows : kSlicedWordRows) && by_rows) sliced = false;
+  uint8_t few_tuned[33] = {0};
+  if (few) {
+    std::lock_guard<std::mutex> lk(g_override_mu);
+    for (uint32_t w = 1; w <= 32; ++w) few_tuned[w] = tuned_by_name(w, batched, n);
+  }
   uint8_t sliced_words[kMaxWords + 1];
   memset(sliced_words, 0, sizeof(sliced_words));
   uint32_t sliced_rows[kSlicedShapes];  // longest length of each bit-sliced shape
@@ -512,7 +528,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   if (sliced) {
     std::lock_guard<std::mutex> lk(g_override_mu);
     for (uint32_t w = kSlicedMinRows / 32 + 1; w <= kSlicedMaxRows / 32; ++w)
-      sliced_words[w] = present[w] && !g_override[batched ? 1 : 0][w].set;
+      sliced_words[w] = present[w] && !g_override[batched ? 1 : 0][w].set && !tuned_by_name(w, batched, n);
   }
   for (uint32_t w = 1; w <= kMaxWords; ++w) {
     if (!present[w]) continue;
@@ -527,7 +543,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     }
     alone = false;
     uint32_t lw = lane_words;
-    if (few && w <= 32) lw = kFewLaneWords;
+    if (few && w <= 32 && !few_tuned[w]) lw = kFewLaneWords;
     else if (small && w <= 32) lw = kSmallBatchLaneWords;
     else if (distinct && w > kDistinctLaneWords && w <= 32) lw = kDistinctLaneWords;
     Shape s = pick_shape(w, batched, lw, large_batch(n));

@@ -59,3 +59,20 @@ def test_admitted_lengths_do_not_depend_on_the_shapes(plan, mode):
         expect = plan(path, lo, hi, n, n // per_read, cut, MYERS_SLICED="0", MYERS_SMALL_BATCH="0")
         for part in expect:
             assert got[part]["admits"] == expect[part]["admits"], (path, lo, hi, n, per_read, cut, part)
+
+
+@pytest.mark.parametrize("path,key", [(PLAIN, "plain"), (BATCHED, "batched"), (BATCHED, "batched_large")])
+def test_named_autotune_file_decides(plan, tmp_path, path, key):
+    """A file that MYERS_AUTOTUNE names decides the shapes of its word counts, in
+    batches of the sizes that take bit-sliced shapes and lanes of few words else."""
+    fn = tmp_path / "tuned.json"
+    entries = {str(w): [16, 2] for w in range(17, 33)}
+    fn.write_text(json.dumps({"plain": {}, "batched": {}, "batched_large": {}} | {key: entries}))
+    other = tmp_path / "other.json"
+    other.write_text(json.dumps({"plain": {}, "batched": {}, "batched_large": {}}))
+    for n in (2_000_000,) if key != "plain" else (2_000_000, 3000):
+        lo, hi = 520, 1000
+        assert all(L == 2 and W == 16 for _, L, W in plan(path, lo, hi, n, n // 11, MYERS_AUTOTUNE=str(fn))["plan"]["shapes"])
+        # word counts that it leaves out are chosen as without it
+        assert plan(path, lo, hi, n, n // 11, MYERS_AUTOTUNE=str(other)) == plan(path, lo, hi, n, n // 11,
+                                                                                 MYERS_AUTOTUNE="0")
