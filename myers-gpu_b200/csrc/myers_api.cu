@@ -1229,7 +1229,7 @@ struct Buffer {
   int last_status;
   bool pending;
   std::vector<uint8_t> present;    // word counts of the last send
-  std::vector<uint8_t> present_m;  // query lengths of the last send (cut-off only)
+  std::vector<uint8_t> present_m;  // query lengths of the last send (scan_lengths)
   PlanTable plan, plan2;
   bool plan_valid;
   int plan_path;
@@ -1378,6 +1378,7 @@ extern "C" int myersInit(void*** myersBuffer, uint32_t numBuffers, const char* r
     const char* g = getenv("MYERS_GRAPHS");
     b->use_graphs = !(g && strcmp(g, "0") == 0);
     b->present.assign(kMaxWords + 1, 0);
+    b->present_m.assign(kMaxWords * 32 + 1, 0);
     bufs[i] = b;
     st = buffer_alloc(b);
     if (st != MYERS_SUCCESS) {
@@ -1396,6 +1397,58 @@ extern "C" int initMyers(void*** myersBuffer, uint32_t numBuffers, const char* r
   return 0;
 }
 
+// Empty queries and those that are too long (flagged on the device) are left out.
+// Without a branch that a length decides: of many queries each length is marked in
+// a table, which then tells the word counts and both ends (two of 50K queries took
+// 27 us to mark their words alone, 55 to 140 with a running minimum and maximum
+// behind branches, and take 21); of few, the table would cost more than it saves.
+// Runs of one length are skipped eight at a time (50K equal ones: 27 -> 18 us).
+Lengths myers::scan_lengths(const qryInfo_t* queries, uint32_t n, uint8_t* present, uint8_t* present_m, bool by_length) {
+  constexpr uint32_t most = kMaxWords * 32;
+  memset(present, 0, kMaxWords + 1);
+  if (!by_length && n < 2048) {
+    uint32_t lo = ~0u, hi = 0;
+    for (uint32_t q = 0; q < n; ++q) {
+      const uint32_t m = queries[q].size;
+      const bool in = m - 1u < most;
+      present[in ? (m + 31) / 32 : 0] = 1;
+      lo = in && m < lo ? m : lo;
+      hi = in && m > hi ? m : hi;
+    }
+    present[0] = 0;
+    return Lengths{hi ? lo : 0, hi};
+  }
+  memset(present_m, 0, most + 1);
+  for (uint32_t q = 0, last = 0; q < n;) {
+    if (q + 8 <= n) {
+      uint32_t other = 0;
+      for (uint32_t k = 0; k < 8; ++k) other |= queries[q + k].size ^ last;
+      if (other == 0) {
+        q += 8;
+        continue;
+      }
+    }
+    for (const uint32_t end = n - q < 128 ? n : q + 128; q < end; ++q) {
+      const uint32_t m = queries[q].size;
+      present_m[m <= most ? m : 0] = 1;
+    }
+    last = queries[q - 1].size;
+  }
+  present_m[0] = 0;
+  Lengths lengths;
+  for (uint32_t w = 1; w <= kMaxWords; ++w) {
+    uint64_t marks[4];
+    memcpy(marks, present_m + 32 * (w - 1) + 1, 32);
+    if (!(marks[0] | marks[1] | marks[2] | marks[3])) continue;
+    present[w] = 1;
+    if (lengths.hi == 0)
+      for (lengths.lo = 32 * (w - 1) + 1; !present_m[lengths.lo];) ++lengths.lo;
+    lengths.hi = 32 * w;
+  }
+  while (lengths.hi && !present_m[lengths.hi]) --lengths.hi;
+  return lengths;
+}
+
 extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint32_t numQueries,
                          uint32_t numCandidates) {
   Buffer* b = static_cast<Buffer*>(mb);
@@ -1406,32 +1459,17 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
     return b->last_status = MYERS_E_CAPACITY;
   NvtxRange range("myers: send");
   CU(cudaSetDevice(b->device));
-  // O(queries) host pass: the word counts present pick the shapes
+  // O(queries) host pass: the lengths present pick the shapes
   std::vector<uint8_t>& present = b->present;
   const bool two_pass = b->cutoff >= 0.0f;
-  Lengths lengths;
-  std::fill(present.begin(), present.end(), 0);
-  for (uint32_t q = 0, last = 0; q < numQueries; ++q) {
-    const uint32_t m = b->h_qinfo[q].size;
-    if (m == last || m > kMaxWords * 32) continue;  // seen, or empty, or too long (flagged on the device)
-    last = m;
-    present[(m + 31) / 32] = 1;
-    if (lengths.lo == 0 || m < lengths.lo) lengths.lo = m;
-    if (m > lengths.hi) lengths.hi = m;
-  }
+  const Lengths lengths = scan_lengths(b->h_qinfo, numQueries, present.data(), b->present_m.data(), two_pass);
   PlanTable& plan = b->plan;
   const uint32_t parts = two_pass || b->in_stream == nullptr ? 1u : send_parts(numCandidates, lengths.hi);
   int st;
   {
     NvtxRange plan_range("myers: send: shape plan");
     if (two_pass) {
-      std::vector<uint8_t>& pm = b->present_m;
-      pm.assign(kMaxWords * 32 + 1, 0);
-      for (uint32_t q = 0; q < numQueries; ++q) {
-        const uint32_t m = b->h_qinfo[q].size;
-        if (m > 0 && m <= kMaxWords * 32) pm[m] = 1;
-      }
-      st = cutoff_plans(plan, b->plan2, pm.data(), b->cutoff, cutoff_prefix_mult(), b->path == MYERS_PATH_BATCHED,
+      st = cutoff_plans(plan, b->plan2, b->present_m.data(), b->cutoff, cutoff_prefix_mult(), b->path == MYERS_PATH_BATCHED,
                         numCandidates);
     } else {
       Batch batch;

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include "../../include/myers-interface.h"
+
 namespace myers {
 
 // An NVTX range over a scope: host stages show up by name on a profiler's
@@ -313,6 +315,10 @@ struct Batch {
   bool unshared = true;   // no other batches share the device (a server's do)
 };
 int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane_words, const Batch& b);
+// The lengths of n queries: the shortest and longest of 1..kMaxWords * 32 bases,
+// their word counts in present[0..kMaxWords] and, where there are many queries or
+// by_length asks for it, each length in present_m[0..kMaxWords * 32].
+Lengths scan_lengths(const qryInfo_t* queries, uint32_t n, uint8_t* present, uint8_t* present_m, bool by_length);
 // The plan of a call whose queries have minSize..maxSize bases (0, 0: any).
 int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.

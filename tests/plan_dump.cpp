@@ -1,6 +1,8 @@
 // Prints the plan that a verify call would take, and the query lengths it
 // admits, without a GPU: plan_dump <path 0|1> <min> <max> <candidates> <reads>
-// <cut-off or -1> (min and max 0: no range announced).
+// <cut-off or -1> (min and max 0: no range announced). Or the lengths that a send
+// sees in its queries, which are the given ones over and over: plan_dump lengths
+// <queries> <mark each length 0|1> <length> <length> ..
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -41,7 +43,25 @@ static void print(const char* name, const PlanTable& p, bool unbucketed) {
   printf("]}");
 }
 
+static int lengths(int argc, char** argv) {
+  const uint32_t n = (uint32_t)atoi(argv[2]);
+  const bool by_length = atoi(argv[3]) != 0;
+  std::vector<qryInfo_t> queries(n);
+  for (uint32_t q = 0; q < n; ++q) queries[q] = qryInfo_t{0, (uint32_t)strtoul(argv[4 + q % (argc - 4)], nullptr, 10)};
+  std::vector<uint8_t> present(kMaxWords + 1, 7), present_m(kMaxWords * 32 + 1, 7);
+  const Lengths l = scan_lengths(queries.data(), n, present.data(), present_m.data(), by_length);
+  printf("{\"lo\": %u, \"hi\": %u, \"words\": [", l.lo, l.hi);
+  for (uint32_t w = 0, any = 0; w <= kMaxWords; ++w)
+    if (present[w]) printf("%s%u", any++ ? ", " : "", w);
+  printf("], \"marked\": [");
+  for (uint32_t m = 0, any = 0; by_length && m <= kMaxWords * 32; ++m)
+    if (present_m[m]) printf("%s%u", any++ ? ", " : "", m);
+  printf("]}\n");
+  return 0;
+}
+
 int main(int argc, char** argv) {
+  if (argc > 4 && strcmp(argv[1], "lengths") == 0) return lengths(argc, argv);
   if (argc != 7) return 2;
   const bool batched = atoi(argv[1]) != 0;
   const uint32_t lo = (uint32_t)atoi(argv[2]), hi = (uint32_t)atoi(argv[3]);

@@ -22,10 +22,14 @@ def plan(tmp_path_factory):
                     f"-Wl,-rpath,{PKG}"], check=True)
 
     def dump(path, lo, hi, n, reads=0, cut=-1.0, **env):
+        return run([path, lo, hi, n, reads, cut], env)
+
+    def run(args, env):
         env = {k: v for k, v in os.environ.items() if not k.startswith("MYERS_")} | env
-        out = subprocess.run([exe, str(path), str(lo), str(hi), str(n), str(reads), str(cut)], env=env, check=True,
-                             capture_output=True, text=True)
+        out = subprocess.run([exe, *map(str, args)], env=env, check=True, capture_output=True, text=True)
         return json.loads(out.stdout)
+
+    dump.lengths = lambda n, by_length, lengths: run(["lengths", n, int(by_length), *lengths], {})
     return dump
 
 
@@ -76,3 +80,18 @@ def test_named_autotune_file_decides(plan, tmp_path, path, key):
         # word counts that it leaves out are chosen as without it
         assert plan(path, lo, hi, n, n // 11, MYERS_AUTOTUNE=str(other)) == plan(path, lo, hi, n, n // 11,
                                                                                  MYERS_AUTOTUNE="0")
+
+
+@pytest.mark.parametrize("lengths", [[100, 200, 0, 1000], [0, 1000, 100], [1000, 1000, 0], [0, 0, 64], [0], [32768, 32769, 1],
+                                     [4294967295, 40000, 33], [0, 65, 64, 0, 96, 97], [5] * 40 + [0, 9] + [7] * 33])
+@pytest.mark.parametrize("n", [1, 7, 8, 129, 2047, 2048, 5003])
+def test_lengths_of_a_send(plan, n, lengths):
+    """Empty queries and those that are too long leave no trace in what the shapes
+    are chosen from, wherever they stand."""
+    there = {(lengths * (n // len(lengths) + 1))[q] for q in range(n)}
+    kept = sorted(m for m in there if 1 <= m <= 32768)
+    for by_length in (False, True):
+        got = plan.lengths(n, by_length, lengths)
+        assert [got["lo"], got["hi"]] == ([kept[0], kept[-1]] if kept else [0, 0])
+        assert got["words"] == sorted({(m + 31) // 32 for m in kept})
+        assert got["marked"] == (kept if by_length else [])
