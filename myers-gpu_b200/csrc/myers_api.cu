@@ -354,7 +354,7 @@ static int sliced_force() {
 //  * the plain path's one-lane shapes of more than 16 words, and its launch per
 //    shape, need as many candidates: 1,000 bases 3.3K 0.67 -> 0.52; 35..301
 //    bases 5K 0.24 -> 0.13, 50K 0.42 -> 0.16 (spread twice; 0.26 unspread).
-static bool sliced_batch(Lengths len, bool batched, uint64_t n, uint32_t& spread) {
+static bool sliced_batch(Lengths len, bool batched, uint64_t n, uint32_t sms, uint32_t& spread) {
   spread = 0;
   if (sliced_force() == 0 || len.hi < kSlicedMinRows || len.lo > kSlicedMaxRows) return false;
   if (sliced_force() < 0 && n < 4096) return false;
@@ -363,7 +363,7 @@ static bool sliced_batch(Lengths len, bool batched, uint64_t n, uint32_t& spread
   int lg, R, lg_lo, R_lo;
   const bool one = sliced_shape(lo, 0, &lg_lo, &R_lo) == sliced_shape(hi, 0, &lg, &R);
   const uint64_t per = 32u << (lg < 5 ? 5 - lg : 0), nw = lg > 5 ? 1u << (lg - 5) : 1u;
-  const uint64_t round = 148u * (uint64_t)kSlicedWarps[sliced_class(Shape{kSlicedVariant, (uint8_t)lg, (uint8_t)R, 0})] / nw;
+  const uint64_t round = sms * (uint64_t)kSlicedWarps[sliced_class(Shape{kSlicedVariant, (uint8_t)lg, (uint8_t)R, 0})] / nw;
   const uint64_t tiles = (n + per - 1) / per;
   if (sliced_force() > 0) {
     spread = (uint32_t)sliced_force() - 1u;
@@ -496,7 +496,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   // of a word count that is present (lengths the caller did not announce but
   // whose word count occurs are admitted, as by the word-parallel shapes).
   bool sliced = lane_words == 0 && (!few || sliced_force() > 0) &&
-                sliced_batch(lengths, batched, b.sliced_n ? b.sliced_n : n, t.spread);
+                sliced_batch(lengths, batched, b.sliced_n ? b.sliced_n : n, b.sms, t.spread);
   // the rows admitted
   const bool adapts = few || sliced;
   uint32_t row_min = 32 * (w_lo - 1) + 1, row_limit = 32 * w_hi, one_rows = 0;
@@ -727,7 +727,7 @@ uint32_t myers::host_prefix_rows(uint32_t m, float cutoff, float mult) {
 }
 
 int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* present_m, float cutoff, float mult,
-                        bool batched, uint64_t n) {
+                        bool batched, uint64_t n, uint32_t sms) {
   uint8_t w1[kMaxWords + 1], w2[kMaxWords + 1];
   memset(w1, 0, sizeof(w1));
   memset(w2, 0, sizeof(w2));
@@ -752,6 +752,7 @@ int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* presen
   auto both = [&](bool bucketed) {
     Batch b;
     b.n = n;
+    b.sms = sms;
     b.lengths = m1;
     b.bucketed = bucketed;
     b.by_words = by_words;
@@ -949,7 +950,8 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
   return MYERS_SUCCESS;
 }
 
-int myers::plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads) {
+int myers::plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads,
+                          uint32_t sms) {
   uint8_t present[kMaxWords + 1];
   memset(present, 0, sizeof(present));
   if (maxSize == 0) maxSize = kMaxWords * 32;
@@ -959,6 +961,7 @@ int myers::plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, i
   Batch b;
   b.n = n;
   b.reads = reads;
+  b.sms = sms;
   b.lengths = Lengths{minSize ? minSize : 1, maxSize};
   return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, b);
 }
@@ -1023,10 +1026,11 @@ static int verify_range(myersContext_t* ctx, const myersReference_t* ref, const 
     std::vector<uint8_t> present_m(kMaxWords * 32 + 1, 0);
     const uint32_t hi = (maxQuerySize == 0 || maxQuerySize > kMaxWords * 32) ? kMaxWords * 32 : maxQuerySize;
     for (uint32_t m = minQuerySize ? minQuerySize : 1; m <= hi; ++m) present_m[m] = 1;
-    st = cutoff_plans(plan, plan2, present_m.data(), cutoff, mult, path == MYERS_PATH_BATCHED, numCandidates);
+    st = cutoff_plans(plan, plan2, present_m.data(), cutoff, mult, path == MYERS_PATH_BATCHED, numCandidates,
+                      (uint32_t)ctx->num_sms);
     if (st == MYERS_SUCCESS) st = ensure_cutoff_scratch(ctx);
   } else {
-    st = plan_for_range(plan, minQuerySize, maxQuerySize, path, numCandidates, numQueries);
+    st = plan_for_range(plan, minQuerySize, maxQuerySize, path, numCandidates, numQueries, (uint32_t)ctx->num_sms);
   }
   if (st != MYERS_SUCCESS) return st;
   DevInputs in;
@@ -1470,12 +1474,13 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
     NvtxRange plan_range("myers: send: shape plan");
     if (two_pass) {
       st = cutoff_plans(plan, b->plan2, b->present_m.data(), b->cutoff, cutoff_prefix_mult(), b->path == MYERS_PATH_BATCHED,
-                        numCandidates);
+                        numCandidates, (uint32_t)b->ctx->num_sms);
     } else {
       Batch batch;
       batch.n = numCandidates / parts;
       batch.reads = numQueries / parts;
       batch.lengths = lengths;
+      batch.sms = (uint32_t)b->ctx->num_sms;
       st = build_plan(plan, present.data(), b->path == MYERS_PATH_BATCHED, 0, batch);
     }
   }
@@ -1725,7 +1730,8 @@ extern "C" int myersVerifyNoAllocAsync(const uint32_t* d_refWords, uint64_t refW
   int st = noalloc_setup(&dev);
   if (st != MYERS_SUCCESS) return st;
   PlanTable plan;
-  st = plan_for_range(plan, minQuerySize, maxQuerySize, MYERS_PATH_BATCHED, numCandidates, numQueries);
+  st = plan_for_range(plan, minQuerySize, maxQuerySize, MYERS_PATH_BATCHED, numCandidates, numQueries,
+                      (uint32_t)dev.num_sms);
   if (st != MYERS_SUCCESS) return st;
   BucketState* d_state = reinterpret_cast<BucketState*>(dev.scratch);
   uint32_t* d_ids = reinterpret_cast<uint32_t*>(dev.scratch + kNoAllocIdsOffset);

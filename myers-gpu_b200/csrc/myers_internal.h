@@ -307,6 +307,7 @@ struct Lengths {
 struct Batch {
   uint64_t n = 0;         // candidates
   uint64_t reads = 0;     // reads they come from (0: unknown)
+  uint32_t sms = 0;       // multiprocessors of the device
   Lengths lengths;        // the shortest and longest query that can occur; with them, large batches take
                           // bit-sliced shapes
   uint64_t sliced_n = 0;  // candidates expected, where they are not n (the cut-off's second pass)
@@ -320,7 +321,8 @@ int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane
 // by_length asks for it, each length in present_m[0..kMaxWords * 32].
 Lengths scan_lengths(const qryInfo_t* queries, uint32_t n, uint8_t* present, uint8_t* present_m, bool by_length);
 // The plan of a call whose queries have minSize..maxSize bases (0, 0: any).
-int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads);
+int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads,
+                   uint32_t sms);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.
 uint32_t batched_tile_bound(const PlanTable& plan, uint32_t n);
 // Record a CUDA failure (message for myersGetErrorString) and return MYERS_E_CUDA.
@@ -367,7 +369,7 @@ int verify_enqueue(myersContext* ctx, const myersReference* ref, const DevInputs
 // first pass's prefix shapes into `plan`, the full-length shapes into
 // `plan2`. `present_m[m]` flags each query length m (1..kMaxWords*32).
 int cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* present_m, float cutoff, float prefix_mult,
-                 bool batched, uint64_t n);
+                 bool batched, uint64_t n, uint32_t sms);
 // The first pass's rows of a query of m bases (as prefix_rows on the device).
 uint32_t host_prefix_rows(uint32_t m, float cutoff, float prefix_mult);
 // Device scratch of the cut-off's second pass for a context (once).

@@ -21,8 +21,8 @@ def plan(tmp_path_factory):
                     os.path.join(ROOT, "tests", "plan_dump.cpp"), os.path.join(PKG, "libmyers_b200.so"),
                     f"-Wl,-rpath,{PKG}"], check=True)
 
-    def dump(path, lo, hi, n, reads=0, cut=-1.0, **env):
-        return run([path, lo, hi, n, reads, cut], env)
+    def dump(path, lo, hi, n, reads=0, cut=-1.0, sms=148, **env):
+        return run([path, lo, hi, n, reads, cut, sms], env)
 
     def run(args, env):
         env = {k: v for k, v in os.environ.items() if not k.startswith("MYERS_")} | env
@@ -95,3 +95,12 @@ def test_lengths_of_a_send(plan, n, lengths):
         assert [got["lo"], got["hi"]] == ([kept[0], kept[-1]] if kept else [0, 0])
         assert got["words"] == sorted({(m + 31) // 32 for m in kept})
         assert got["marked"] == (kept if by_length else [])
+
+
+def test_rounds_are_those_of_the_device(plan):
+    """Half the multiprocessors take the shapes of twice the candidates."""
+    for lo, hi in ((400, 400), (1000, 1000), (3000, 3000), (100, 1000)):
+        for n in range(20_000, 400_000, 20_000):
+            whole, half = plan(BATCHED, lo, hi, n), plan(BATCHED, lo, hi, n // 2, sms=74)
+            if n // 2 >= 150_000 or n < 150_000:  # on one side of the table for large batches
+                assert whole["plan"]["sliced"] == half["plan"]["sliced"], (lo, hi, n)
