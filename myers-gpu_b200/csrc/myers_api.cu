@@ -305,19 +305,35 @@ static bool small_batch(uint64_t n) {
   return n > 0 && n < threshold;
 }
 
+static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words = 0, bool large = false);
+
 // Whether a batch is so small that the time of one tile counts, not the lanes'
 // efficiency: reads of up to 1,024 bases then take lanes of kFewLaneWords words
-// on either path. The batch's
-// words per column are estimated from the word counts that occur, 0.6 of the
-// middle where they differ. Measured on the batched path, against lanes of 12
-// words: 1,000 bases 110 candidates 0.21 -> 0.15 ms, 11K 0.46 -> 0.42, 22K 0.71 ->
-// 0.82; 400 bases 11K 0.151 -> 0.124, 33K 0.25 -> 0.27; 100..1,000 bases 1.1K 0.21 ->
-// 0.15, 11K 0.46 -> 0.29, 33K 0.46 -> 0.36, 66K 0.61 -> 0.63. On the plain path,
-// against one lane of 32 words: 1,000 bases 110 candidates 0.50 -> 0.14 ms.
+// on either path. The batch's words per column are estimated from the word counts
+// that occur, 0.6 of the middle where they differ (from its PEQ entries, if that
+// is more, where no range is announced).
+// Against lanes of 12 words on the batched path: 1,000 bases 110 candidates 0.21 ->
+// 0.15 ms, 100..1,000 bases 1.1K 0.21 -> 0.15, 11K 0.46 -> 0.29, 33K 0.46 -> 0.36,
+// 66K 0.61 -> 0.63; against one lane of 32 words on the plain path: 1,000 bases 110
+// candidates 0.50 -> 0.14.
+//
+// Between these limits both sides run whole waves, a tile per scheduler at a time.
+// On the batched path a column takes 45 ns and, for each tile that a scheduler
+// runs, 10.6 W + 6 ns for lanes of W words (within 5% for W = 4 .. 12 and up to
+// four tiles; five of W = 5 take a sixth more), so one length compares these: 760
+// bases 3.3K candidates 0.18 -> 0.11 ms (1 wave of tiles each), 7.7K 0.18 -> 0.23 (3
+// against 1), 9.9K 0.31 -> 0.23 (3 against 2). Mixed lengths blur the waves, except
+// for the second one against a first (500..1,000 bases 5K 0.28 -> 0.30) and where
+// the lengths are close (900..1,000 bases 12K 0.53 -> 0.45, 20K 0.66 -> 0.71).
+// On the plain path the one-lane shapes of 17, 19 and 20 words run a column in 265,
+// 216 and 216 ns (18: 313), and hold out up to three and two waves (600 bases 11K
+// 0.185 -> 0.188, 16.5K 0.185 -> 0.24).
+//
 // Not in the serving loop, whose slots fill the device together: there 64
 // requests gained (733 -> 592 us), but 86M candidates/s offered had a p99 of
 // 3.6-8.4 ms instead of 1.6-2.3, and of 1.7-5.3 with a quarter of the threshold.
-static bool few_words(const uint8_t* present, uint64_t n) {
+static bool few_words(const uint8_t* present, bool batched, const Batch& b) {
+  const uint64_t n = b.n;
   if (!small_batch(n)) return false;
   uint32_t lo = 0, hi = 0;
   for (uint32_t w = 1; w <= 32; ++w)
@@ -325,7 +341,39 @@ static bool few_words(const uint8_t* present, uint64_t n) {
       if (lo == 0) lo = w;
       hi = w;
     }
-  return hi >= kFewMinWords && n * (lo == hi ? 10ull * hi : 3ull * (lo + hi)) < 10ull * kFewWords;
+  if (hi < kFewMinWords) return false;
+  uint64_t tenths = lo == hi ? 10ull * hi : 3ull * (lo + hi);  // of a word
+  const bool any_length = batched && b.any_length;
+  if (any_length && b.mean > 0) {
+    const uint64_t mean = b.mean >= 1024 ? 320 : b.mean * 10ull / 32;
+    if (mean > tenths) tenths = mean;
+  }
+  if (n * tenths >= 10ull * kFewWords) return false;
+  const uint64_t slots = 4ull * b.sms;  // schedulers: a tile on each is a wave
+  auto waves = [&](double tiles) { return (uint64_t)(tiles / (double)slots) + 1; };
+  auto lanes = [&](uint32_t w, uint32_t lane_words) { return pick_shape(w, batched, w > lane_words ? lane_words : 0); };
+  auto per = [](Shape s) { return variant_multi(s.variant) ? 32u / s.L : 32u; };
+  if (!batched) {
+    const uint64_t most = hi == 17 ? 3 : hi == 19 || hi == 20 ? 2 : 0;
+    return lo != hi || most == 0 || waves((double)(n - 1) / per(lanes(hi, kFewLaneWords))) <= most;
+  }
+  if (lo == hi) {
+    const Shape f = lanes(hi, kFewLaneWords), s = lanes(hi, kSmallBatchLaneWords);
+    const uint64_t wf = waves((double)(n - 1) / per(f)), ws = waves((double)(n - 1) / per(s));
+    return (wf < 5 || f.W == 4) && wf * (106u * f.W + 60u) < ws * (106u * s.W + 60u);
+  }
+  if (any_length) return true;
+  if (hi < 2 * lo && n * tenths >= 7ull * kFewWords) return false;
+  // lengths spread evenly over their logarithm
+  if (n <= 4 * slots) return true;  // one wave at least four candidates to a tile
+  double tf = 0, ts = 0, sum = 0;
+  for (uint32_t w = lo; w <= hi; ++w)
+    if (present[w]) {
+      sum += 1.0 / w;
+      tf += 1.0 / w / per(lanes(w, kFewLaneWords));
+      ts += 1.0 / w / per(lanes(w, kSmallBatchLaneWords));
+    }
+  return !(waves(tf / sum * (double)n) == 2 && waves(ts / sum * (double)n) == 1);
 }
 
 // MYERS_SLICED=0 turns the bit-sliced shapes off; 1 takes them for every batch, 2
@@ -338,47 +386,103 @@ static int sliced_force() {
   return force;
 }
 
-// Whether a batch of n candidates of queries of lo..hi bases takes bit-sliced
-// shapes (myers_sliced.cuh) for those of kSlicedMinRows..kSlicedMaxRows bases,
-// and how far it spreads them. A tile of theirs is 32 candidates or more on one
-// warp (on two to eight warps beyond 1,024 bases), so a batch has to fill the
-// device with such tiles. Measured, word-parallel against bit-sliced:
-//  * one length, which ends with whole rounds of tiles: 1,000 bases 33K
-//    candidates (0.87 of a round) 0.98 -> 0.82 ms, 660K 17.3 -> 12.5; 400 bases
-//    330K 1.50 -> 1.17; 100 bases 330K (1.1 rounds) 0.159 -> 0.152, 1.1M 0.446 ->
-//    0.38; 3,000 bases 11K (1.16 rounds) 3.1 -> 3.6, 44K 11.7 -> 8.5; 8,000
-//    bases 4.4K (0.93) 8.6 -> 6.0;
-//  * mixed lengths, where a round of the longest tiles comes on top: 100..1,000
-//    bases 33K 0.46 -> 0.58, 110K (2.9 rounds of the longest) 0.93 -> 0.89, 220K
-//    1.73 -> 1.35; 1,000..10,000 bases 15K 10.9 -> 11.2, 40K 25.9 -> 18.6;
-//  * the plain path's one-lane shapes of more than 16 words, and its launch per
-//    shape, need as many candidates: 1,000 bases 3.3K 0.67 -> 0.52; 35..301
-//    bases 5K 0.24 -> 0.13, 50K 0.42 -> 0.16 (spread twice; 0.26 unspread).
-static bool sliced_batch(Lengths len, bool batched, uint64_t n, uint32_t sms, uint32_t& spread) {
+// Tiles of n candidates of m bases in their bit-sliced shape, and how many of them
+// the device runs at a time.
+struct SlicedTiles {
+  uint64_t tiles, round;
+  int lg, R;
+};
+static SlicedTiles sliced_tiles(uint32_t m, uint64_t n, uint32_t sms) {
+  SlicedTiles t;
+  sliced_shape(m, 0, &t.lg, &t.R);
+  const uint64_t per = 32u << (t.lg < 5 ? 5 - t.lg : 0), warps = t.lg > 5 ? 1u << (t.lg - 5) : 1u;
+  t.round = sms * (uint64_t)kSlicedWarps[sliced_class(Shape{kSlicedVariant, (uint8_t)t.lg, (uint8_t)t.R, 0})] / warps;
+  t.tiles = (n + per - 1) / per;
+  return t;
+}
+
+// Whether a batch takes bit-sliced shapes (myers_sliced.cuh) for its queries of
+// kSlicedMinRows..kSlicedMaxRows bases, and how far it spreads them. A tile of
+// theirs is 32 candidates or more on one warp (on two to eight warps beyond 1,024
+// bases), so a batch has to fill the device with such tiles. Below, in ms, the
+// word-parallel shapes and the bit-sliced ones.
+static bool sliced_batch(const Batch& b, bool batched, uint32_t& spread) {
   spread = 0;
+  const Lengths len = b.lengths;
+  const uint64_t n = b.sliced_n ? b.sliced_n : b.n;
   if (sliced_force() == 0 || len.hi < kSlicedMinRows || len.lo > kSlicedMaxRows) return false;
-  if (sliced_force() < 0 && n < 4096) return false;
-  const uint32_t lo = len.lo < kSlicedMinRows ? kSlicedMinRows : len.lo;
-  const uint32_t hi = len.hi > kSlicedMaxRows ? kSlicedMaxRows : len.hi;
-  int lg, R, lg_lo, R_lo;
-  const bool one = sliced_shape(lo, 0, &lg_lo, &R_lo) == sliced_shape(hi, 0, &lg, &R);
-  const uint64_t per = 32u << (lg < 5 ? 5 - lg : 0), nw = lg > 5 ? 1u << (lg - 5) : 1u;
-  const uint64_t round = sms * (uint64_t)kSlicedWarps[sliced_class(Shape{kSlicedVariant, (uint8_t)lg, (uint8_t)R, 0})] / nw;
-  const uint64_t tiles = (n + per - 1) / per;
   if (sliced_force() > 0) {
     spread = (uint32_t)sliced_force() - 1u;
     return true;
   }
-  // Reads of many short lengths are a round of every class of shapes: doubled
-  // tiles shorten them while they stay within some rounds (300K reads of 35..301
-  // bases 0.41 -> 0.36 ms, 150K 0.34 -> 0.26).
-  if (!one && lg < 5)
+  if (n < 4096) return false;
+  const uint32_t lo = len.lo < kSlicedMinRows ? kSlicedMinRows : len.lo;
+  const uint32_t hi = len.hi > kSlicedMaxRows ? kSlicedMaxRows : len.hi;
+  const SlicedTiles t = sliced_tiles(hi, n, b.sms);
+  const uint64_t tiles = t.tiles, round = t.round, rounds = (tiles + round - 1) / round;
+  int lg, R;
+  if (len.lo >= kSlicedMinRows && sliced_shape(lo, 0, &lg, &R) == sliced_shape(hi, 0, &lg, &R)) {
+    // One length, which ends with whole rounds of tiles: 1,000 bases 33K
+    // candidates (0.87 of a round) 0.98 -> 0.82, 660K 17.3 -> 12.5; 400 bases 330K
+    // 1.50 -> 1.17; 3,000 bases 11K (1.16 rounds) 3.1 -> 3.6, 44K 11.7 -> 8.5; 8,000
+    // bases 4.4K (0.93) 8.6 -> 6.0.
+    const bool filled = rounds >= 4 || 10 * tiles >= 7 * rounds * round;
+    if (hi <= 512 && rounds < 2) return false;
+    if (batched) return filled;
+    // On the plain path one lane holds up to 1,024 bases without bucketing. Few
+    // words run near the ALU's limit, the nearer the fuller the last word: 66 bases
+    // 660K 0.157 -> 0.162, 96 bases 0.207 -> 0.222, 900K 0.278 -> 0.288, 100 bases 660K
+    // 0.271 -> 0.242, 128 bases 0.336 -> 0.340, 900K (3 rounds) 0.453 -> 0.431, 160
+    // bases 330K (1.5 rounds) 0.254 -> 0.274, 440K (1.9) 0.347 -> 0.322.
+    if (hi <= 96) return false;
+    if (hi > 120 && hi <= 128) return filled && 10 * tiles >= 25 * round;
+    if (hi > 136 && hi <= 160) return filled && 10 * tiles >= 19 * round;
+    // Shapes of 17 to 32 words need many candidates for a wave of their own, which
+    // ends with four, and again with seven tiles per multiprocessor: 1,000 bases 3.3K
+    // 0.67 -> 0.52, 600 bases 16K (four) 0.19 -> 0.28, 24K 0.36 -> 0.33, 33K (seven) 0.36
+    // -> 0.45, 38K 0.53 -> 0.45.
+    if (hi > 512 && hi <= 1024 && rounds <= 1)
+      return hi > 768 || (tiles > 4ull * b.sms && tiles <= 6ull * b.sms) || tiles > 7ull * b.sms;
+    return filled;
+  }
+  // Mixed lengths, where a round of the longest tiles comes on top. Reads of many
+  // short lengths are a round of every class of shapes: doubled tiles shorten them
+  // while they stay within some rounds (300K reads of 35..301 bases 0.41 -> 0.36 ms,
+  // 150K 0.34 -> 0.26).
+  if (t.lg < 5)
     while (spread < 2 && (tiles << (spread + 1)) <= kSpreadRounds * round) ++spread;
-  if (!one) return 4 * tiles >= 11 * round || (!batched && hi <= 1024);
-  const uint64_t rounds = (tiles + round - 1) / round;
-  if (!batched && hi > 512 && hi <= 1024 && rounds <= 1) return true;
-  if (hi <= 512 && rounds < 2) return false;
-  return rounds >= 4 || 10 * tiles >= 7 * rounds * round;
+  const bool close = 2 * (uint64_t)len.hi <= 5 * (uint64_t)len.lo;
+  if (!batched) {
+    // The plain path launches every word count by itself, each with a tail: 35..301
+    // bases 5K 0.21 -> 0.11, 500K 0.66 -> 0.51, 1M 0.82 -> 0.88 (its launches are full
+    // then); 40..200 bases 330K 0.35 -> 0.27, 500K 0.36 -> 0.39; 65..512 bases 750K
+    // 1.89 -> 1.55, 1M 2.08 -> 2.14; 250..500 bases 1.3M 5.1 -> 4.1; 65..128 bases 5K
+    // 0.064 -> 0.088, 60K 0.115 -> 0.107, 220K 0.148 -> 0.165.
+    if (hi > 1024) return 4 * tiles >= 11 * round;
+    if (hi > 512 || (hi > 256 && close)) return true;
+    if (hi <= 128) return len.lo >= kSlicedMinRows && n >= 100ull * b.sms && n <= 1000ull * b.sms;
+    return 2 * n <= 23ull * hi * b.sms;
+  }
+  // On the batched path one launch carries every word-parallel shape. Without a range
+  // the mean read says what the batch holds: 50K candidates of 100 bases 0.16 -> 0.21
+  // and 35..301 bases 0.25 -> 0.57 without this, 1,000 bases 110K 3.3 -> 2.4 with it.
+  if (b.any_length || (b.mean > 0 && len.hi > 8 * b.mean)) {
+    if (b.mean < 256) return false;
+    const SlicedTiles m = sliced_tiles(b.mean > kSlicedMaxRows ? kSlicedMaxRows : (uint32_t)b.mean, n, b.sms);
+    return 4 * m.tiles >= 11 * m.round;
+  }
+  // Reads of up to 64 bases, or of more than 10,240, keep that launch, and the
+  // bit-sliced ones follow it: 35..301 bases 400K 0.36 -> 0.51, 1.3M 1.10 -> 1.17,
+  // 20..1,000 bases 120K (3.2 rounds) 0.82 -> 0.88, 220K 1.10 -> 1.09; 1,000..12,000
+  // bases 20K (4.2 rounds) 18.2 -> 19.3, 25K 22.6 -> 19.4.
+  if (len.lo < kSlicedMinRows || len.hi > kSlicedMaxRows) return len.hi > 512 && tiles >= 5 * round;
+  // 70..150 bases 660K 0.37 -> 0.38; 65..512 bases 750K 1.49 -> 1.57, 200..400 bases
+  // 500K 1.35 -> 1.26, 100..1,000 bases 110K (2.9 rounds) 0.93 -> 0.89; 1,000..10,000
+  // bases 15K (3.2 rounds) 10.9 -> 12.0, 25K 16.9 -> 12.2, 3,000..6,000 bases 15K 9.3 ->
+  // 7.3.
+  if (hi <= 256 || (hi <= 768 && !close)) return false;
+  if (hi > 1024 && len.hi > 4 * len.lo) return tiles >= 4 * round;
+  return 4 * tiles >= 11 * round;
 }
 
 // Fewer than two candidates per read (0 reads: unknown).
@@ -388,7 +492,7 @@ static bool few_candidates(uint64_t n, uint64_t reads) { return reads > 0 && n <
 // lane_words words is spread over ceil(words / W) lanes of W <= lane_words
 // words, the cheapest such shape by the cost model (shorter per-candidate
 // time, some more instructions). `large`: the batch is large (large_batch).
-static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words = 0, bool large = false) {
+static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words, bool large) {
   load_tuned_once();
   {
     std::lock_guard<std::mutex> lk(g_override_mu);
@@ -486,7 +590,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     }
   if (w_lo == 0) return MYERS_SUCCESS;
   const bool small = batched && lane_words == 0 && small_batch(n);
-  const bool few = b.unshared && few_words(present, n);
+  const bool few = b.unshared && lane_words == 0 && few_words(present, batched, b);
   // Fewer than two candidates per read: a warp of 32 one-lane candidates then
   // holds more distinct reads than the 16 PEQ slots of the single-lane shapes
   // of more than 16 words, and runs its lanes in two rounds. Lanes of at most
@@ -496,7 +600,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   // of a word count that is present (lengths the caller did not announce but
   // whose word count occurs are admitted, as by the word-parallel shapes).
   bool sliced = lane_words == 0 && (!few || sliced_force() > 0) &&
-                sliced_batch(lengths, batched, b.sliced_n ? b.sliced_n : n, b.sms, t.spread);
+                sliced_batch(b, batched, t.spread);
   // the rows admitted
   const bool adapts = few || sliced;
   uint32_t row_min = 32 * (w_lo - 1) + 1, row_limit = 32 * w_hi, one_rows = 0;
@@ -727,7 +831,7 @@ uint32_t myers::host_prefix_rows(uint32_t m, float cutoff, float mult) {
 }
 
 int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* present_m, float cutoff, float mult,
-                        bool batched, uint64_t n, uint32_t sms) {
+                        bool batched, uint64_t n, uint32_t sms, uint32_t mean, bool any_length) {
   uint8_t w1[kMaxWords + 1], w2[kMaxWords + 1];
   memset(w1, 0, sizeof(w1));
   memset(w2, 0, sizeof(w2));
@@ -753,11 +857,14 @@ int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* presen
     Batch b;
     b.n = n;
     b.sms = sms;
+    b.any_length = any_length;
+    b.mean = mean ? host_prefix_rows(mean, cutoff, mult) : 0;
     b.lengths = m1;
     b.bucketed = bucketed;
     b.by_words = by_words;
     const int st = build_plan(plan, w1, batched, 0, b);
     b.reads = n;
+    b.mean = mean;
     b.lengths = m2;
     b.sliced_n = n / 8;
     return st != MYERS_SUCCESS ? st : build_plan(plan2, w2, batched, 0, b);
@@ -950,10 +1057,19 @@ int myers::verify_enqueue(myersContext* ctx, const myersReference* ref, const De
   return MYERS_SUCCESS;
 }
 
+// Bases of a read on average, as far as its PEQ entries tell: half an entry short of
+// them (0: unknown).
+static uint32_t mean_bases(uint64_t entries, uint64_t reads) {
+  if (reads == 0) return 0;
+  const uint64_t m = entries * NUM_BASES_ENTRY / reads;
+  return m <= NUM_BASES_ENTRY / 2 ? 1u : (uint32_t)(m < kMaxWords * 32 ? m - NUM_BASES_ENTRY / 2 : kMaxWords * 32);
+}
+
 int myers::plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads,
-                          uint32_t sms) {
+                          uint64_t entries, uint32_t sms) {
   uint8_t present[kMaxWords + 1];
   memset(present, 0, sizeof(present));
+  const bool any_length = maxSize == 0;
   if (maxSize == 0) maxSize = kMaxWords * 32;
   if (maxSize > kMaxWords * 32) maxSize = kMaxWords * 32;
   const uint32_t wlo = minSize ? (minSize + 31) / 32 : 1, whi = (maxSize + 31) / 32;
@@ -962,6 +1078,8 @@ int myers::plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, i
   b.n = n;
   b.reads = reads;
   b.sms = sms;
+  b.any_length = any_length;
+  b.mean = mean_bases(entries, reads);
   b.lengths = Lengths{minSize ? minSize : 1, maxSize};
   return build_plan(plan, present, path == MYERS_PATH_BATCHED, 0, b);
 }
@@ -1027,10 +1145,11 @@ static int verify_range(myersContext_t* ctx, const myersReference_t* ref, const 
     const uint32_t hi = (maxQuerySize == 0 || maxQuerySize > kMaxWords * 32) ? kMaxWords * 32 : maxQuerySize;
     for (uint32_t m = minQuerySize ? minQuerySize : 1; m <= hi; ++m) present_m[m] = 1;
     st = cutoff_plans(plan, plan2, present_m.data(), cutoff, mult, path == MYERS_PATH_BATCHED, numCandidates,
-                      (uint32_t)ctx->num_sms);
+                      (uint32_t)ctx->num_sms, mean_bases(numPEQEntries, numQueries), maxQuerySize == 0);
     if (st == MYERS_SUCCESS) st = ensure_cutoff_scratch(ctx);
   } else {
-    st = plan_for_range(plan, minQuerySize, maxQuerySize, path, numCandidates, numQueries, (uint32_t)ctx->num_sms);
+    st = plan_for_range(plan, minQuerySize, maxQuerySize, path, numCandidates, numQueries, numPEQEntries,
+                        (uint32_t)ctx->num_sms);
   }
   if (st != MYERS_SUCCESS) return st;
   DevInputs in;
@@ -1474,7 +1593,7 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
     NvtxRange plan_range("myers: send: shape plan");
     if (two_pass) {
       st = cutoff_plans(plan, b->plan2, b->present_m.data(), b->cutoff, cutoff_prefix_mult(), b->path == MYERS_PATH_BATCHED,
-                        numCandidates, (uint32_t)b->ctx->num_sms);
+                        numCandidates, (uint32_t)b->ctx->num_sms, 0, false);
     } else {
       Batch batch;
       batch.n = numCandidates / parts;
@@ -1730,7 +1849,7 @@ extern "C" int myersVerifyNoAllocAsync(const uint32_t* d_refWords, uint64_t refW
   int st = noalloc_setup(&dev);
   if (st != MYERS_SUCCESS) return st;
   PlanTable plan;
-  st = plan_for_range(plan, minQuerySize, maxQuerySize, MYERS_PATH_BATCHED, numCandidates, numQueries,
+  st = plan_for_range(plan, minQuerySize, maxQuerySize, MYERS_PATH_BATCHED, numCandidates, numQueries, numPEQEntries,
                       (uint32_t)dev.num_sms);
   if (st != MYERS_SUCCESS) return st;
   BucketState* d_state = reinterpret_cast<BucketState*>(dev.scratch);

@@ -310,6 +310,8 @@ struct Batch {
   uint32_t sms = 0;       // multiprocessors of the device
   Lengths lengths;        // the shortest and longest query that can occur; with them, large batches take
                           // bit-sliced shapes
+  bool any_length = false;  // the caller announced no range of lengths
+  uint32_t mean = 0;      // bases of a read on average (0: unknown)
   uint64_t sliced_n = 0;  // candidates expected, where they are not n (the cut-off's second pass)
   bool bucketed = false;  // the candidates will be classified in any case: name every shape of the word counts present
   bool by_words = false;  // admit queries by their word counts alone
@@ -322,7 +324,7 @@ int build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32_t lane
 Lengths scan_lengths(const qryInfo_t* queries, uint32_t n, uint8_t* present, uint8_t* present_m, bool by_length);
 // The plan of a call whose queries have minSize..maxSize bases (0, 0: any).
 int plan_for_range(PlanTable& plan, uint32_t minSize, uint32_t maxSize, int path, uint64_t n, uint64_t reads,
-                   uint32_t sms);
+                   uint64_t entries, uint32_t sms);
 // Upper bound of the persistent kernel's tiles for n candidates under `plan`.
 uint32_t batched_tile_bound(const PlanTable& plan, uint32_t n);
 // Record a CUDA failure (message for myersGetErrorString) and return MYERS_E_CUDA.
@@ -367,9 +369,10 @@ int verify_enqueue(myersContext* ctx, const myersReference* ref, const DevInputs
                    cudaStream_t s, const PlanTable* plan2 = nullptr);
 // The cut-off's plans from the word counts of the full queries present: the
 // first pass's prefix shapes into `plan`, the full-length shapes into
-// `plan2`. `present_m[m]` flags each query length m (1..kMaxWords*32).
+// `plan2`. `present_m[m]` flags each query length m (1..kMaxWords*32); mean and
+// any_length as in Batch.
 int cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* present_m, float cutoff, float prefix_mult,
-                 bool batched, uint64_t n, uint32_t sms);
+                 bool batched, uint64_t n, uint32_t sms, uint32_t mean, bool any_length);
 // The first pass's rows of a query of m bases (as prefix_rows on the device).
 uint32_t host_prefix_rows(uint32_t m, float cutoff, float prefix_mult);
 // Device scratch of the cut-off's second pass for a context (once).

@@ -1,6 +1,6 @@
 // Prints the plan that a verify call would take, and the query lengths it
 // admits, without a GPU: plan_dump <path 0|1> <min> <max> <candidates> <reads>
-// <cut-off or -1> [multiprocessors, else 148] (min and max 0: no range announced). Or the lengths that a send
+// <cut-off or -1> <multiprocessors> <PEQ entries> (min and max 0: no range announced). Or the lengths that a send
 // sees in its queries, which are the given ones over and over: plan_dump lengths
 // <queries> <mark each length 0|1> <length> <length> ..
 #include <cstdint>
@@ -62,8 +62,9 @@ static int lengths(int argc, char** argv) {
 
 int main(int argc, char** argv) {
   if (argc > 4 && strcmp(argv[1], "lengths") == 0) return lengths(argc, argv);
-  if (argc != 7 && argc != 8) return 2;
-  const uint32_t sms = argc == 8 ? (uint32_t)atoi(argv[7]) : 148;
+  if (argc != 9) return 2;
+  const uint32_t sms = (uint32_t)atoi(argv[7]);
+  const uint64_t entries = strtoull(argv[8], nullptr, 10);
   const bool batched = atoi(argv[1]) != 0;
   const uint32_t lo = (uint32_t)atoi(argv[2]), hi = (uint32_t)atoi(argv[3]);
   const uint64_t n = strtoull(argv[4], nullptr, 10), reads = strtoull(argv[5], nullptr, 10);
@@ -75,7 +76,7 @@ int main(int argc, char** argv) {
   if (cut >= 0.0f) {
     std::vector<uint8_t> present(kMaxWords * 32 + 1, 0);
     for (uint32_t m = first; m <= last; ++m) present[m] = 1;
-    if (cutoff_plans(a, b, present.data(), cut, cutoff_prefix_mult(), batched, n, sms) != 0) return 1;
+    if (cutoff_plans(a, b, present.data(), cut, cutoff_prefix_mult(), batched, n, sms, 0, hi == 0) != 0) return 1;
     const bool unbucketed = !batched && !a.bucketed;
     printf("{");
     print("first", a, unbucketed);
@@ -84,7 +85,7 @@ int main(int argc, char** argv) {
     printf("}\n");
     return 0;
   }
-  if (plan_for_range(a, lo, hi, batched, n, reads, sms) != 0) return 1;
+  if (plan_for_range(a, lo, hi, batched, n, reads, entries, sms) != 0) return 1;
   const bool unbucketed = sliced_alone(a) || (!batched && a.num_cfg == 1 && a.num_sliced == 0);
   printf("{");
   print("plan", a, unbucketed);

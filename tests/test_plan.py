@@ -21,8 +21,8 @@ def plan(tmp_path_factory):
                     os.path.join(ROOT, "tests", "plan_dump.cpp"), os.path.join(PKG, "libmyers_b200.so"),
                     f"-Wl,-rpath,{PKG}"], check=True)
 
-    def dump(path, lo, hi, n, reads=0, cut=-1.0, sms=148, **env):
-        return run([path, lo, hi, n, reads, cut, sms], env)
+    def dump(path, lo, hi, n, reads=0, cut=-1.0, sms=148, entries=0, **env):
+        return run([path, lo, hi, n, reads, cut, sms, entries], env)
 
     def run(args, env):
         env = {k: v for k, v in os.environ.items() if not k.startswith("MYERS_")} | env
@@ -104,3 +104,44 @@ def test_rounds_are_those_of_the_device(plan):
             whole, half = plan(BATCHED, lo, hi, n), plan(BATCHED, lo, hi, n // 2, sms=74)
             if n // 2 >= 150_000 or n < 150_000:  # on one side of the table for large batches
                 assert whole["plan"]["sliced"] == half["plan"]["sliced"], (lo, hi, n)
+
+
+# path, lengths, candidates, reads, PEQ entries (0, 0: a range is announced) and whether bit-sliced shapes are faster
+SLICED = [(PLAIN, 66, 66, 660_000, 0, 0, False), (PLAIN, 96, 96, 520_000, 0, 0, False), (PLAIN, 100, 100, 660_000, 0, 0, True),
+          (PLAIN, 128, 128, 440_000, 0, 0, False), (PLAIN, 160, 160, 330_000, 0, 0, False),
+          (PLAIN, 160, 160, 440_000, 0, 0, True), (PLAIN, 600, 600, 33_000, 0, 0, False),
+          (PLAIN, 600, 600, 38_000, 0, 0, True), (PLAIN, 600, 600, 16_500, 0, 0, False), (PLAIN, 600, 600, 24_000, 0, 0, True), (PLAIN, 20, 120, 60_000, 0, 0, False), (PLAIN, 20, 120, 660_000, 0, 0, False),
+          (PLAIN, 65, 128, 5_000, 0, 0, False), (PLAIN, 35, 301, 5_000, 0, 0, True), (PLAIN, 35, 301, 300_000, 0, 0, True),
+          (PLAIN, 35, 301, 1_300_000, 0, 0, False), (PLAIN, 250, 500, 1_300_000, 0, 0, True),
+          (BATCHED, 35, 301, 660_000, 0, 0, False), (BATCHED, 35, 512, 660_000, 0, 0, False),
+          (BATCHED, 20, 1000, 120_000, 0, 0, False), (BATCHED, 100, 1000, 110_000, 0, 0, True),
+          (BATCHED, 1000, 10_000, 15_000, 0, 0, False), (BATCHED, 3000, 6000, 15_000, 0, 0, True),
+          (BATCHED, 1000, 10_000, 100_000, 0, 0, True), (BATCHED, 1000, 12_000, 15_000, 0, 0, False),
+          (BATCHED, 0, 0, 50_000, 4545, 4545, False), (BATCHED, 0, 0, 300_000, 27_272, 27_272, False),
+          (BATCHED, 0, 0, 110_000, 10_000, 14_000, False), (BATCHED, 0, 0, 110_000, 10_000, 80_000, True)]
+
+
+@pytest.mark.parametrize("path,lo,hi,n,reads,entries,faster", SLICED)
+def test_bit_sliced_where_it_is_faster(plan, path, lo, hi, n, reads, entries, faster):
+    assert (plan(path, lo, hi, n, reads, entries=entries)["plan"]["sliced"] > 0) == faster
+
+
+@pytest.mark.parametrize("m,n,faster", [(760, 3300, True), (760, 7700, False), (760, 9900, True), (760, 16_500, False),
+                                        (880, 3300, False), (880, 5500, True), (1000, 3300, False), (1000, 5500, True),
+                                        (1000, 7700, False), (400, 5500, True), (400, 7700, False), (400, 9900, True)])
+def test_lanes_of_few_words_where_they_are_faster(plan, m, n, faster):
+    p = plan(BATCHED, m, m, n)["plan"]
+    assert (p["shapes"][0][2] <= 5) == faster
+
+
+@pytest.mark.parametrize("m,n,faster", [(600, 9000, True), (600, 16_500, False), (560, 16_500, True), (1000, 12_000, True)])
+def test_lanes_of_few_words_on_the_plain_path(plan, m, n, faster):
+    p = plan(PLAIN, m, m, n)["plan"]
+    assert (p["shapes"][0][2] <= 5) == faster
+
+
+@pytest.mark.parametrize("entries,faster", [(1272 * 8, False), (1272 * 2, True)])
+def test_lanes_of_few_words_without_a_range(plan, entries, faster):
+    """14K candidates of 1,000 and of 200 bases."""
+    p = plan(BATCHED, 0, 0, 14_000, 1272, entries=entries)["plan"]
+    assert all(W <= 5 for v, L, W in p["shapes"] if 32 * L * W in range(400, 1024)) == faster
