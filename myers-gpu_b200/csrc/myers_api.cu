@@ -576,19 +576,20 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
   memset(t.cfg_of_sliced, kNoCfg, sizeof(t.cfg_of_sliced));
   Shape shapes[kMaxCfg];
   uint32_t max_words[kMaxCfg];
-  int16_t cfg_of[kMaxWords + 1];
+  uint8_t cfg_of[kMaxWords + 1];
   int nshapes = 0;
-  for (uint32_t w = 0; w <= kMaxWords; ++w) cfg_of[w] = -1;
   const uint64_t n = b.n;
   const Lengths lengths = b.lengths;
   t.bucketed = b.bucketed;
-  uint32_t w_lo = 0, w_hi = 0;
-  for (uint32_t w = 1; w <= kMaxWords; ++w)
-    if (present[w]) {
-      if (w_lo == 0) w_lo = w;
-      w_hi = w;
-    }
-  if (w_lo == 0) return MYERS_SUCCESS;
+  uint32_t w_lo = 1, w_hi = kMaxWords;
+  while (w_lo <= kMaxWords && !present[w_lo]) ++w_lo;
+  if (w_lo > kMaxWords) return MYERS_SUCCESS;
+  for (uint64_t eight; w_hi >= w_lo + 8; w_hi -= 8) {
+    memcpy(&eight, present + w_hi - 7, 8);
+    if (eight) break;
+  }
+  while (!present[w_hi]) --w_hi;
+  memset(cfg_of + w_lo, kNoCfg, w_hi - w_lo + 1);
   const bool small = batched && lane_words == 0 && small_batch(n);
   const bool few = b.unshared && lane_words == 0 && few_words(present, batched, b);
   // Fewer than two candidates per read: a warp of 32 one-lane candidates then
@@ -617,9 +618,7 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     for (uint32_t w = 1; w <= 32; ++w) few_tuned[w] = tuned_by_name(w, batched, n);
   }
   uint8_t sliced_words[kMaxWords + 1];
-  memset(sliced_words, 0, sizeof(sliced_words));
   uint32_t sliced_rows[kSlicedShapes];  // longest length of each bit-sliced shape
-  memset(sliced_rows, 0, sizeof(sliced_rows));
   // every length that can occur has the same bit-sliced shape (a longer length
   // never has a smaller one): one shape for every candidate, so no bucketing
   bool alone = sliced && !b.bucketed && lengths.lo >= kSlicedMinRows && lengths.hi <= kSlicedMaxRows;
@@ -630,13 +629,15 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
     alone = alone_shape == sliced_shape(lengths.hi, t.spread, &lg, &R);
   }
   if (sliced) {
+    memset(sliced_words, 0, sizeof(sliced_words));
+    memset(sliced_rows, 0, sizeof(sliced_rows));
     std::lock_guard<std::mutex> lk(g_override_mu);
     for (uint32_t w = kSlicedMinRows / 32 + 1; w <= kSlicedMaxRows / 32; ++w)
       sliced_words[w] = present[w] && !g_override[batched ? 1 : 0][w].set && !tuned_by_name(w, batched, n);
   }
-  for (uint32_t w = 1; w <= kMaxWords; ++w) {
+  for (uint32_t w = w_lo; w <= w_hi; ++w) {
     if (!present[w]) continue;
-    if (sliced_words[w]) {
+    if (sliced && sliced_words[w]) {
       t.cfg_of_words[w] = kSlicedCfg;
       for (uint32_t m = 32 * (w - 1) + 1; m <= 32 * w; ++m) {
         int lg, R;
@@ -663,9 +664,9 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
       found = nshapes++;
     }
     if (w > max_words[found]) max_words[found] = w;
-    cfg_of[w] = (int16_t)found;
+    cfg_of[w] = (uint8_t)found;
   }
-  for (int i = 0; i < kSlicedShapes; ++i) {
+  for (int i = 0; sliced && i < kSlicedShapes; ++i) {
     if (sliced_rows[i] == 0 || (alone && i != alone_shape)) continue;
     if (nshapes == kMaxCfg) return MYERS_E_QUERY_TOO_LONG;
     int lg, R;
@@ -715,8 +716,8 @@ int myers::build_plan(PlanTable& t, const uint8_t* present, bool batched, uint32
       t.cfg_of_sliced[sliced_shape(max_words[order[r]], t.spread, &lg, &R)] = (uint8_t)r;
     }
   }
-  for (uint32_t w = 1; w <= kMaxWords; ++w)
-    if (cfg_of[w] >= 0) t.cfg_of_words[w] = (uint8_t)rank[cfg_of[w]];
+  for (uint32_t w = w_lo; w <= w_hi; ++w)
+    if (cfg_of[w] != kNoCfg) t.cfg_of_words[w] = (uint8_t)rank[cfg_of[w]];
   if (by_rows && (b.bucketed || nshapes > 1)) {
     // Shorter lengths than those present fit the first one's shape; longer ones go
     // to the last one's, which verifies them up to row_limit and flags the rest.

@@ -114,25 +114,30 @@ __host__ __device__ inline int sliced_shape(uint32_t m, uint32_t spread, int* lg
   return (g - kSlicedMinLg) * (kSlicedMaxR - kSlicedMinR + 1) + r - kSlicedMinR;
 }
 
-// Per-send plan, passed by value as a __grid_constant__ kernel parameter:
-// word count -> shape index, and the shapes in launch order. The first
+// Per-send plan, its two parts passed by value as __grid_constant__ kernel
+// parameters, each to the kernels that read it (with one table for all of them,
+// the four launches of a small batch took 1.6 us more on the host): word count ->
+// shape index for the classification, and the shapes in launch order. The first
 // num_batched shapes (most expensive first) go to the persistent kernel on
 // the batched path, the next num_sliced to the bit-sliced kernel on both
 // paths; the rest always get plain launches.
-struct PlanTable {
+struct PlanLookup {
   uint8_t cfg_of_words[kMaxWords + 1];
   uint8_t cfg_of_sliced[kSlicedShapes];
+  uint32_t spread;     // of the bit-sliced shapes
+};
+struct PlanShapes {
   uint32_t num_cfg;
   uint32_t num_batched;
   uint32_t num_sliced;
-  uint32_t spread;     // of the bit-sliced shapes
   uint32_t bucketed;   // the candidates are to be classified, also where there is one shape
   uint32_t row_min, row_limit;  // the rows admitted (0, 0: what the shapes hold)
   Shape shape[kMaxCfg];
 };
+struct PlanTable : PlanLookup, PlanShapes {};
 
 // The shape of m rows (1..kMaxWords * 32) under a plan, or kNoCfg.
-__host__ __device__ inline uint32_t plan_cfg(const PlanTable& plan, uint32_t m) {
+__host__ __device__ inline uint32_t plan_cfg(const PlanLookup& plan, uint32_t m) {
   const uint32_t c = plan.cfg_of_words[(m + 31) >> 5];
   if (c != kSlicedCfg) return c;
   if (m < kSlicedMinRows || m > kSlicedMaxRows) return kNoCfg;
@@ -254,19 +259,19 @@ constexpr int kSlicedWarps[kSlicedClasses] = {16, 12, 8, 8};  // warps per SM
 // candidates 0..count-1 as shape c0, with the tile counter d_next (zero when
 // the launch starts).
 template <int CLASS>
-cudaError_t launch_sliced_class(const DevInputs& in, const uint32_t* d_ids, const PlanTable& plan, BucketState* d_state,
+cudaError_t launch_sliced_class(const DevInputs& in, const uint32_t* d_ids, const PlanShapes& plan, BucketState* d_state,
                                 uint32_t c0, uint32_t c1, uint32_t count, uint32_t* d_next, cudaStream_t s, int num_sms);
 template <int CLASS>
 const void* sliced_class_kernel();
-template <> cudaError_t launch_sliced_class<0>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
-template <> cudaError_t launch_sliced_class<1>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
-template <> cudaError_t launch_sliced_class<2>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
-template <> cudaError_t launch_sliced_class<3>(const DevInputs&, const uint32_t*, const PlanTable&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> cudaError_t launch_sliced_class<0>(const DevInputs&, const uint32_t*, const PlanShapes&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> cudaError_t launch_sliced_class<1>(const DevInputs&, const uint32_t*, const PlanShapes&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> cudaError_t launch_sliced_class<2>(const DevInputs&, const uint32_t*, const PlanShapes&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
+template <> cudaError_t launch_sliced_class<3>(const DevInputs&, const uint32_t*, const PlanShapes&, BucketState*, uint32_t, uint32_t, uint32_t, uint32_t*, cudaStream_t, int);
 template <> const void* sliced_class_kernel<0>();
 template <> const void* sliced_class_kernel<1>();
 template <> const void* sliced_class_kernel<2>();
 template <> const void* sliced_class_kernel<3>();
-inline cudaError_t launch_sliced(int cls, const DevInputs& in, const uint32_t* d_ids, const PlanTable& plan,
+inline cudaError_t launch_sliced(int cls, const DevInputs& in, const uint32_t* d_ids, const PlanShapes& plan,
                                  BucketState* d_state, uint32_t c0, uint32_t c1, uint32_t count, uint32_t* d_next,
                                  cudaStream_t s, int num_sms) {
   switch (cls) {

@@ -75,8 +75,16 @@ __global__ void __launch_bounds__(128) k_plain(DevInputs in, const uint32_t* __r
 // its query, by its full word count under `plan2` into in.esc_cfg, counted in
 // in.esc_state->cursor (the second pass's layout).
 template <bool TWO>
-__global__ void k_classify(DevInputs in, const __grid_constant__ PlanTable plan,
-                           const __grid_constant__ PlanTable plan2, BucketState* st,
+struct Lookups {
+  PlanLookup plan, second;
+};
+template <>
+struct Lookups<false> {
+  PlanLookup plan;
+};
+
+template <bool TWO>
+__global__ void k_classify(DevInputs in, const __grid_constant__ Lookups<TWO> plans, BucketState* st,
                            uint8_t* __restrict__ cfg_of_cand) {
   const int lane = threadIdx.x & 31;
   const uint32_t n = in.num_cands;
@@ -102,16 +110,21 @@ __global__ void k_classify(DevInputs in, const __grid_constant__ PlanTable plan,
         in.results[i] = make_uint2(0u, kNoResult);
       } else if (m == 0) {
         in.results[i] = make_uint2(0u, 0u);
-      } else if (mf > kMaxWords * 32 || ncol > kMaxColumns || plan_cfg(plan, m) == kNoCfg ||
-                 (TWO && m < mf && plan_cfg(plan2, mf) == kNoCfg)) {
-        in.results[i] = make_uint2(0u, kNoResult);
-        atomicOr(in.flags, kFlagUnsupported);
       } else {
-        cfg = plan_cfg(plan, m);
-        if (TWO && m < mf) {
-          const uint32_t c2 = plan_cfg(plan2, mf);
-          in.esc_cfg[i] = (uint8_t)c2;
-          atomicAdd(&in.esc_state->cursor[c2], 1u);
+        const bool sized = mf <= kMaxWords * 32 && ncol <= kMaxColumns;
+        uint32_t second = 0;
+        if (sized) {
+          cfg = plan_cfg(plans.plan, m);
+          if constexpr (TWO)
+            if (m < mf) second = plan_cfg(plans.second, mf);
+        }
+        if (cfg == kNoCfg || second == kNoCfg) {
+          cfg = kNoCfg;
+          in.results[i] = make_uint2(0u, kNoResult);
+          atomicOr(in.flags, kFlagUnsupported);
+        } else if (TWO && m < mf) {
+          in.esc_cfg[i] = (uint8_t)second;
+          atomicAdd(&in.esc_state->cursor[second], 1u);
         }
       }
       cfg_of_cand[i] = (uint8_t)cfg;
@@ -124,7 +137,7 @@ __global__ void k_classify(DevInputs in, const __grid_constant__ PlanTable plan,
 // The second pass's layout: each full-length shape's list starts where the
 // candidates counted for it in the classification end up at most; the lists
 // fill as the first pass appends to them.
-__global__ void k_plan_escalation(const __grid_constant__ PlanTable plan2, BucketState* esc) {
+__global__ void k_plan_escalation(const __grid_constant__ PlanShapes plan2, BucketState* esc) {
   if (threadIdx.x != 0) return;
   uint32_t acc = 0;
   for (uint32_t c = 0; c < plan2.num_cfg; ++c) {
@@ -138,7 +151,7 @@ __global__ void k_plan_escalation(const __grid_constant__ PlanTable plan2, Bucke
 // The second pass's tiles on the persistent path, once the first pass has
 // filled the lists: each shape's tiles from its list length, the persistent
 // kernel's tile count and a fresh work counter.
-__global__ void k_plan_tiles(const __grid_constant__ PlanTable plan2, BucketState* esc) {
+__global__ void k_plan_tiles(const __grid_constant__ PlanShapes plan2, BucketState* esc) {
   if (threadIdx.x != 0) return;
   uint32_t tiles = 0;
   for (uint32_t c = 0; c < plan2.num_cfg; ++c) {
@@ -153,7 +166,7 @@ __global__ void k_plan_tiles(const __grid_constant__ PlanTable plan2, BucketStat
   esc->queue = 0;
 }
 
-__global__ void k_plan(const __grid_constant__ PlanTable plan, BucketState* st) {
+__global__ void k_plan(const __grid_constant__ PlanShapes plan, BucketState* st) {
   if (threadIdx.x != 0) return;
   uint32_t acc = 0, tiles = 0;
   for (uint32_t c = 0; c < plan.num_cfg; ++c) {
@@ -230,7 +243,7 @@ __device__ __forceinline__ void dispatch(int v, const DevInputs& in, const uint3
 #define MYERS_BATCHED_MIN_BLOCKS 3
 #endif
 __global__ void __launch_bounds__(128, MYERS_BATCHED_MIN_BLOCKS) k_batched(DevInputs in, const uint32_t* __restrict__ ids,
-                                                 const __grid_constant__ PlanTable plan, BucketState* st) {
+                                                 const __grid_constant__ PlanShapes plan, BucketState* st) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint32_t s_tile_start[kMaxCfg + 1];
   __shared__ uint32_t s_first[kMaxCfg];
@@ -349,7 +362,7 @@ int launch_bucketing(const DevInputs& in, const PlanTable& plan, BucketState* d_
   const uint32_t need = (in.num_cands + threads - 1) / threads;
   uint32_t grid = (uint32_t)num_sms * 8;
   if (need < grid) grid = need > 0 ? need : 1;
-  k_classify<false><<<grid, threads, 0, s>>>(in, plan, plan, d_state, d_cfg_of_cand);
+  k_classify<false><<<grid, threads, 0, s>>>(in, Lookups<false>{plan}, d_state, d_cfg_of_cand);
   k_plan<<<1, 32, 0, s>>>(plan, d_state);
   k_scatter<<<grid, threads, 0, s>>>(in.num_cands, d_cfg_of_cand, d_state, d_ids);
   *err = cudaGetLastError();
@@ -363,7 +376,7 @@ int launch_bucketing_cutoff(const DevInputs& in, const PlanTable& plan, const Pl
   const uint32_t need = (in.num_cands + threads - 1) / threads;
   uint32_t grid = (uint32_t)num_sms * 8;
   if (need < grid) grid = need > 0 ? need : 1;
-  k_classify<true><<<grid, threads, 0, s>>>(in, plan, plan2, d_state, d_cfg_of_cand);
+  k_classify<true><<<grid, threads, 0, s>>>(in, Lookups<true>{plan, plan2}, d_state, d_cfg_of_cand);
   k_plan<<<1, 32, 0, s>>>(plan, d_state);
   k_plan_escalation<<<1, 32, 0, s>>>(plan2, in.esc_state);
   k_scatter<<<grid, threads, 0, s>>>(in.num_cands, d_cfg_of_cand, d_state, d_ids);

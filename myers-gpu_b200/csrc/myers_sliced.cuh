@@ -597,7 +597,7 @@ __device__ __forceinline__ void run_tile(const DevInputs& in, const Tile& t, int
 template <class K>
 __global__ void __launch_bounds__(K::kThreads, K::kBlocks)
     k_sliced(const __grid_constant__ DevInputs in, const uint32_t* __restrict__ ids, BucketState* st,
-             const __grid_constant__ PlanTable plan, uint32_t c0, uint32_t c1, uint32_t count,
+             const __grid_constant__ PlanShapes plan, uint32_t c0, uint32_t c1, uint32_t count,
              uint32_t* __restrict__ next) {
   __shared__ uint32_t s_tile[K::kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(K::kThreads, K::kBlocks)
 }
 
 template <class K>
-cudaError_t launch_class(const DevInputs& in, const uint32_t* d_ids, const PlanTable& plan, BucketState* d_state,
+cudaError_t launch_class(const DevInputs& in, const uint32_t* d_ids, const PlanShapes& plan, BucketState* d_state,
                          uint32_t c0, uint32_t c1, uint32_t count, uint32_t* d_next, cudaStream_t s, int num_sms) {
   cudaError_t e = cudaFuncSetAttribute((const void*)k_sliced<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)K::kSmemBytes);
@@ -710,7 +710,7 @@ cudaError_t launch_class(const DevInputs& in, const uint32_t* d_ids, const PlanT
 // compiled in a file of its own: together they take minutes.
 #define MYERS_SLICED_CLASS(K, INDEX)                                                                                 \
   template <>                                                                                                        \
-  cudaError_t launch_sliced_class<INDEX>(const DevInputs& in, const uint32_t* d_ids, const PlanTable& plan,          \
+  cudaError_t launch_sliced_class<INDEX>(const DevInputs& in, const uint32_t* d_ids, const PlanShapes& plan,          \
                                          BucketState* d_state, uint32_t c0, uint32_t c1, uint32_t count,             \
                                          uint32_t* d_next, cudaStream_t s, int num_sms) {                            \
     return launch_class<K>(in, d_ids, plan, d_state, c0, c1, count, d_next, s, num_sms);                             \

@@ -398,6 +398,11 @@ __device__ __forceinline__ uint32_t check_query(const DevInputs& in, uint32_t qu
 // Resolve the candidate of this segment and write the result of candidates
 // that need no DP (window out of range, empty query, unsupported size,
 // invalid indices).
+// BOUNDED: the plan may admit fewer rows than the tile holds (in.row_min,
+// in.row_limit). Not so on one lane per candidate, whose shape is itself what the
+// admitted rows are taken from; the test there cost the two-word shape a block per
+// multiprocessor.
+template <bool BOUNDED>
 __device__ __forceinline__ CandSetup setup_candidate(const DevInputs& in, const uint32_t* __restrict__ ids,
                                                      uint32_t first, uint32_t cnt, int seg, int nseg,
                                                      int l, int rows) {
@@ -427,7 +432,8 @@ __device__ __forceinline__ CandSetup setup_candidate(const DevInputs& in, const 
     const uint32_t wb = d_window_bases(c.mf, in.distance);
     const bool valid = bad == 0u && c.pos < in.ref_size && (in.ref_size - c.pos) > (unsigned long long)wb;
     c.n = in.exact ? wb : 8u * d_window_words(wb);
-    const bool fits = c.m >= in.row_min && c.m <= min((uint32_t)rows, in.row_limit) && c.n <= kMaxColumns;
+    bool fits = c.m <= (uint32_t)rows && c.n <= kMaxColumns;
+    if (BOUNDED) fits = fits && c.m >= in.row_min && c.m <= in.row_limit;
     c.qok = bad == 0u && c.m > 0 && c.m <= (uint32_t)rows;
     c.work = valid && c.m > 0 && fits;
     if (!c.work && l == 0) {
@@ -453,7 +459,7 @@ __device__ __forceinline__ void process_tile(const DevInputs& in, const uint32_t
   const int LW = Lr * W;
   const int rows = 32 * LW;
 
-  const CandSetup c = setup_candidate(in, ids, first, cnt, seg, nseg, l, rows);
+  const CandSetup c = setup_candidate<MULTI>(in, ids, first, cnt, seg, nseg, l, rows);
 
   // One slot per run of segments with the same read: a run starts where the
   // read differs from the previous segment's.

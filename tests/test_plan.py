@@ -49,7 +49,7 @@ def test_bit_sliced_tiles_can_fall_back(plan, tmp_path, words, shape, length):
 
 RANGES = [(1, 32), (35, 301), (65, 96), (100, 100), (100, 128), (20, 1000), (545, 576), (640, 640), (700, 736), (900, 1000),
           (930, 960), (940, 950), (961, 1000), (990, 1000), (1000, 1000), (1000, 1100), (1025, 1088), (1040, 1060),
-          (1500, 1600), (1505, 1568), (2000, 2048), (5000, 5100), (9000, 9600), (10000, 10200), (1000, 12000), (0, 0)]
+          (1500, 1600), (1505, 1568), (2000, 2048), (5000, 5100), (9000, 9600), (10000, 10200), (1000, 12000), (1, 1), (32750, 32768), (0, 0)]
 CALLS = list(itertools.product((PLAIN, BATCHED), RANGES, (100, 3000, 20_000, 120_000, 1_000_000), (1, 11),
                                (-1.0, 0.0, 0.04, 0.2, 1.0)))
 
