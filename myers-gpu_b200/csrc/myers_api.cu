@@ -1668,7 +1668,15 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
     return MYERS_SUCCESS;
   };
   st = b->use_graphs ? launch_as_graph(s, &b->exec, enqueue) : enqueue();
-  if (st != MYERS_SUCCESS) return b->last_status = st;
+  if (st != MYERS_SUCCESS) {
+    if (parts > 1) {
+      // the buffer's stream has not been joined with these, whose copies read and
+      // write the caller's arrays
+      cudaStreamSynchronize(b->in_stream);
+      cudaStreamSynchronize(b->out_stream);
+    }
+    return b->last_status = st;
+  }
   b->pending = true;
   return MYERS_SUCCESS;
 }
