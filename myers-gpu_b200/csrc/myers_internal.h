@@ -103,7 +103,7 @@ constexpr uint32_t kSlicedWordRows = 4096, kSlicedChainWordRows = 16384;
 constexpr int kSlicedShapes = (kSlicedMaxLg - kSlicedMinLg + 1) * (kSlicedMaxR - kSlicedMinR + 1);
 
 // Index of the bit-sliced shape of m rows (kSlicedMinRows..kSlicedMaxRows).
-__host__ __device__ inline int sliced_shape(uint32_t m, uint32_t spread, int* lg, int* R) {
+__host__ __device__ constexpr int sliced_shape(uint32_t m, uint32_t spread, int* lg, int* R) {
   int g = kSlicedMinLg;
   while (g < kSlicedMaxLg && m > (32u << g)) ++g;
   for (; spread > 0 && g < 5 && m > (7u << (g + 1)); --spread) ++g;
