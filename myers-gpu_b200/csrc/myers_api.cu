@@ -1357,9 +1357,8 @@ struct Buffer {
   PlanTable plan, plan2;
   bool plan_valid;
   int plan_path;
-  // streams of a send in parts (send_parts), made by the first such send: copies
-  // in, copies out; null when they could not be made
-  bool part_streams;
+  // streams of a send in parts (send_parts): copies in, copies out; null where the
+  // buffer is too small for one, or when they could not be made
   cudaStream_t in_stream, out_stream;
   cudaEvent_t fork, copied[kSendParts], verified[kSendParts], out_done;
 };
@@ -1390,7 +1389,6 @@ static void part_streams_free(Buffer* b) {
 
 // Without them a send goes through in one part.
 static void part_streams_create(Buffer* b) {
-  b->part_streams = true;
   bool ok = cudaStreamCreateWithFlags(&b->in_stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaStreamCreateWithFlags(&b->out_stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess &&
@@ -1434,6 +1432,7 @@ static int buffer_alloc(Buffer* b) {
 #define ALLOC_D(p, n) \
   if (cudaMalloc((void**)&(p), (size_t)(n) ? (size_t)(n) : 1) != cudaSuccess) return MYERS_E_INSUFFICIENT_MEM_GPU
   CU(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+  if (b->maxCandidates >= 2 * kPartCandidates) part_streams_create(b);
   ALLOC_H(b->h_peq, (size_t)b->maxPEQEntries * sizeof(qryEntry_t));
   ALLOC_H(b->h_qinfo, (size_t)b->maxQueries * sizeof(qryInfo_t));
   ALLOC_H(b->h_cands, (size_t)b->maxCandidates * sizeof(candInfo_t));
@@ -1589,9 +1588,7 @@ extern "C" int myersSend(void* mb, float distance, uint32_t numPEQEntries, uint3
   const bool two_pass = b->cutoff >= 0.0f;
   const Lengths lengths = scan_lengths(b->h_qinfo, numQueries, present.data(), b->present_m.data(), two_pass);
   PlanTable& plan = b->plan;
-  uint32_t parts = two_pass ? 1u : send_parts(numCandidates, lengths.hi);
-  if (parts > 1 && !b->part_streams) part_streams_create(b);
-  if (b->in_stream == nullptr) parts = 1;
+  const uint32_t parts = two_pass || b->in_stream == nullptr ? 1u : send_parts(numCandidates, lengths.hi);
   int st;
   {
     NvtxRange plan_range("myers: send: shape plan");
