@@ -31,7 +31,9 @@ JSON line (rank 0).
             under Ukkonen's cut-off, and a short serving sweep
 
 --impl reference times the reference's own CPU implementation instead (the
-GPU path of the reference targets sm_20..sm_50 only).
+GPU path of the reference targets sm_20..sm_50 only). Where that code is not
+present (oracle/_ref/, built from the reference's sources) the line says
+"unavailable" with the reason.
 """
 import argparse
 import json
@@ -364,19 +366,18 @@ def run_reference(args):
     k = args.workload
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import oracle as orc
+    if not orc.have_reference():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's own CPU code is not built here (oracle/_ref): "
+                                                              "its sources are not on this machine"}), flush=True)
+        return
     threads = host_threads()
-    kind = "reference" if orc.have_reference() else "port"
     per_step = max(1.0, min(10.0, 120.0 / max(1, args.steps + args.warmup)))
     s, ref_words, ref_size, w = make_inputs(ms, k, args.scale, 0, num_reads=max(1, 2000 // (10 if k in (2, 4) else 1)))
-    padded = orc.pad_reference(ref_words) if kind == "reference" else None
+    padded = orc.pad_reference(ref_words)
 
     def run(w):
-        if kind == "reference":
-            return orc.reference_verify_aligned(w["peq"], w["qinfo"], w["cands"], ref_words, ref_size, DIST,
-                                                nthreads=threads, padded=padded)[1]
-        t = time.perf_counter()
-        orc.verify(w["peq"], w["qinfo"], w["cands"], ref_words, ref_size, DIST, nthreads=threads)
-        return time.perf_counter() - t
+        return orc.reference_verify_aligned(w["peq"], w["qinfo"], w["cands"], ref_words, ref_size, DIST,
+                                            nthreads=threads, padded=padded)[1]
 
     sec = max(run(w), 1e-4)
     full = ms.workload_spec(k, scale=args.scale)
@@ -396,12 +397,11 @@ def run_reference(args):
             "data": "synthetic (seeded)", "gcups": float(cells.sum() / t / 1e9),
             "config": {"workload": WORKLOAD_NAMES[k], "candidates_per_gpu": full_cands, "distance": DIST,
                        "window": "aligned",
-                       "path": "the reference's CPU Myers (computeAllQueriesCPU)" if kind == "reference"
-                       else "CPU port of the reference algorithm",
+                       "path": "the reference's CPU Myers (computeAllQueriesCPU)",
                        "l2": "host caches (CPU)", "parallelism": f"{threads} host threads",
                        "sample_candidates_per_step": len(w["cands"]),
                        "sample_fraction": len(w["cands"]) / full_cands},
-            "cpu_baseline": {"value": cps, "unit": "candidates/s", "cores": threads, "kind": kind,
+            "cpu_baseline": {"value": cps, "unit": "candidates/s", "cores": threads, "kind": "reference",
                              "sample": f"each step: first {s.num_reads} reads ({len(w['cands'])} candidates, "
                                        f"{100 * len(w['cands']) / full_cands:.1f}% of the workload), "
                                        f"OpenMP over {threads} threads"},
