@@ -278,7 +278,7 @@ static bool tuned_by_name(uint32_t w, bool batched, uint64_t n) {
   return g_tuned_named && (g_tuned[batched ? 1 : 0][w].set || (batched && large_batch(n) && g_tuned[2][w].set));
 }
 
-// How many of a context's streams the plain path spreads its launches over
+// How many of a context's streams the launches per shape are spread over
 // (MYERS_PLAIN_STREAMS, 1..kPlainStreams; 1 keeps them on the caller's stream).
 static int plain_streams() {
   static const int k = [] {
@@ -764,8 +764,8 @@ extern "C" int myersContextCreate(myersContext_t** out, uint64_t maxCandidates) 
     delete c;
     return e == cudaErrorMemoryAllocation ? MYERS_E_INSUFFICIENT_MEM_GPU : cuda_fail(e, "context");
   }
-  // The plain path's streams. Without them its launches stay on the caller's
-  // stream, one after another.
+  // The streams of the launches per shape. Without them these stay on the
+  // caller's stream, one after another.
   bool streams = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) == cudaSuccess;
   for (int i = 0; i < kPlainStreams && streams; ++i)
     streams = cudaStreamCreateWithFlags(&c->aux[i], cudaStreamNonBlocking) == cudaSuccess &&
@@ -1111,10 +1111,8 @@ extern "C" int myersVerifyRangeAsync(myersContext_t* ctx, const myersReference_t
 // Ukkonen's cut-off (GEMTools/src/gt_map_align_bpm.c:141-210,
 // gt_map_block_bpm_get_distance__cutoff): the result is exact where the
 // minimum is at most (uint32_t)(m * cutoff), else {MYERS_NO_MATCH,
-// MYERS_NO_MATCH}. The plain path's word-parallel single-lane shapes of 8..32
-// words (a multiple of 4) skip the rows above the band; the bit-sliced and the
-// other shapes and the batched path compute every row and apply the same
-// contract.
+// MYERS_NO_MATCH}. On either path a first pass runs a prefix of each query, and
+// the candidates that the prefix does not settle run in full (cutoff_plans).
 extern "C" int myersVerifyCutoffAsync(myersContext_t* ctx, const myersReference_t* ref, const qryEntry_t* d_peq,
                                       uint32_t numPEQEntries, const qryInfo_t* d_qinfo, uint32_t numQueries,
                                       const candInfo_t* d_cands, uint32_t numCandidates, float distance,

@@ -358,8 +358,9 @@ struct myersContext {
   uint32_t* d_esc_ids;
   uint8_t* d_esc_cfg;
   myers::BucketState* d_esc_state;
-  // streams the plain path spreads its per-shape launches over (forked from
-  // and joined back to the caller's stream); null when they could not be made
+  // streams that the launches per shape (on the batched path those beside the
+  // persistent kernel) are spread over, forked from and joined back to the
+  // caller's stream; null when they could not be made
   cudaStream_t aux[myers::kPlainStreams];
   cudaEvent_t fork;
   cudaEvent_t join[myers::kPlainStreams];
