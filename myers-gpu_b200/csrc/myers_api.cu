@@ -323,8 +323,11 @@ static Shape pick_shape(uint32_t w, bool batched, uint32_t lane_words = 0, bool 
 // four tiles; five of W = 5 take a sixth more), so one length compares these: 760
 // bases 3.3K candidates 0.18 -> 0.11 ms (1 wave of tiles each), 7.7K 0.18 -> 0.23 (3
 // against 1), 9.9K 0.31 -> 0.23 (3 against 2). Mixed lengths blur the waves, except
-// for the second one against a first (500..1,000 bases 5K 0.28 -> 0.30) and where
-// the lengths are close (900..1,000 bases 12K 0.53 -> 0.45, 20K 0.66 -> 0.71).
+// for the second one against a first while two lanes of 12 words hold the longest
+// read (410..698 bases 8.4K 0.18 -> 0.24, 216..658 8.7K 0.17 -> 0.22; of three lanes
+// the tiles are too long: 613..916 bases 5.2K 0.33 -> 0.22, 114..824 9.6K 0.36 -> 0.25,
+// 100..1,000 9K 0.32 -> 0.28) and where the lengths are close (900..1,000 bases 12K 0.53
+// -> 0.45, 20K 0.66 -> 0.71).
 // On the plain path the one-lane shapes of 17, 19 and 20 words run a column in 265,
 // 216 and 216 ns (18: 313), and hold out up to three and two waves (600 bases 11K
 // 0.185 -> 0.188, 16.5K 0.185 -> 0.24).
@@ -364,6 +367,7 @@ static bool few_words(const uint8_t* present, bool batched, const Batch& b) {
   }
   if (any_length) return true;
   if (hi < 2 * lo && n * tenths >= 7ull * kFewWords) return false;
+  if (hi > 2 * kSmallBatchLaneWords) return true;
   // lengths spread evenly over their logarithm
   if (n <= 4 * slots) return true;  // one wave at least four candidates to a tile
   double tf = 0, ts = 0, sum = 0;

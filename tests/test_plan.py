@@ -145,3 +145,10 @@ def test_lanes_of_few_words_without_a_range(plan, entries, faster):
     """14K candidates of 1,000 and of 200 bases."""
     p = plan(BATCHED, 0, 0, 14_000, 1272, entries=entries)["plan"]
     assert all(W <= 5 for v, L, W in p["shapes"] if 32 * L * W in range(400, 1024)) == faster
+
+
+@pytest.mark.parametrize("lo,hi,n,faster", [(613, 916, 5176, True), (114, 824, 9583, True), (100, 1000, 9000, True),
+                                            (410, 698, 8447, False), (216, 658, 8746, False)])
+def test_lanes_of_few_words_for_mixed_lengths(plan, lo, hi, n, faster):
+    p = plan(BATCHED, lo, hi, n)["plan"]
+    assert all(W <= 5 for v, L, W in p["shapes"]) == faster
