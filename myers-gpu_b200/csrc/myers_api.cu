@@ -390,6 +390,9 @@ static int sliced_force() {
   return force;
 }
 
+// Fewer than two candidates per read (0 reads: unknown).
+static bool few_candidates(uint64_t n, uint64_t reads) { return reads > 0 && n < 2 * reads; }
+
 // Tiles of n candidates of m bases in their bit-sliced shape, and how many of them
 // the device runs at a time.
 struct SlicedTiles {
@@ -442,11 +445,14 @@ static bool sliced_batch(const Batch& b, bool batched, uint32_t& spread) {
     if (hi > 120 && hi <= 128) return filled && 10 * tiles >= 25 * round;
     if (hi > 136 && hi <= 160) return filled && 10 * tiles >= 19 * round;
     // Shapes of 17 to 32 words need many candidates for a wave of their own, which
-    // ends with four, and again with seven tiles per multiprocessor: 1,000 bases 3.3K
-    // 0.67 -> 0.52, 600 bases 16K (four) 0.19 -> 0.28, 24K 0.36 -> 0.33, 33K (seven) 0.36
-    // -> 0.45, 38K 0.53 -> 0.45.
+    // ends with four, and again with eight tiles per multiprocessor, while bit-sliced
+    // tiles take longer from a little over six: 1,000 bases 3.3K 0.67 -> 0.52, 600 bases
+    // 16K (four) 0.19 -> 0.28, 24K 0.36 -> 0.33, 565 bases 28.7K (6.1) 0.37 -> 0.32, 600
+    // bases 33K (seven) 0.36 -> 0.45, 37K (7.9) 0.36 -> 0.45, 38K 0.53 -> 0.45. A read or
+    // more per candidate, as in the cut-off's second pass, takes two lanes instead: 666
+    // bases 292K, cut-off at 0.04 m, 1.42 -> 1.03.
     if (hi > 512 && hi <= 1024 && rounds <= 1)
-      return hi > 768 || (tiles > 4ull * b.sms && tiles <= 6ull * b.sms) || tiles > 7ull * b.sms;
+      return hi > 768 || few_candidates(n, b.reads) || (tiles > 4ull * b.sms && 10 * tiles <= 63ull * b.sms) || tiles > 8ull * b.sms;
     return filled;
   }
   // Mixed lengths, where a round of the longest tiles comes on top. Reads of many
@@ -479,18 +485,20 @@ static bool sliced_batch(const Batch& b, bool batched, uint32_t& spread) {
   // bit-sliced ones follow it: 35..301 bases 400K 0.36 -> 0.51, 1.3M 1.10 -> 1.17,
   // 20..1,000 bases 120K (3.2 rounds) 0.82 -> 0.88, 220K 1.10 -> 1.09; 1,000..12,000
   // bases 20K (4.2 rounds) 18.2 -> 19.3, 25K 22.6 -> 19.4.
+  // Nor with a read or more of its own per candidate, which short tiles don't hide:
+  // 104..331 bases 1.1M of one read each 1.65 -> 2.51, 217..503 bases 660K 2.37 -> 3.08.
+  if (hi <= 768 && few_candidates(n, b.reads)) return false;
   if (len.lo < kSlicedMinRows || len.hi > kSlicedMaxRows) return len.hi > 512 && tiles >= 5 * round;
-  // 70..150 bases 660K 0.37 -> 0.38; 65..512 bases 750K 1.49 -> 1.57, 200..400 bases
-  // 500K 1.35 -> 1.26, 100..1,000 bases 110K (2.9 rounds) 0.93 -> 0.89; 1,000..10,000
-  // bases 15K (3.2 rounds) 10.9 -> 12.0, 25K 16.9 -> 12.2, 3,000..6,000 bases 15K 9.3 ->
-  // 7.3.
-  if (hi <= 256 || (hi <= 768 && !close)) return false;
-  if (hi > 1024 && len.hi > 4 * len.lo) return tiles >= 4 * round;
+  // 70..150 bases 660K (2.2 rounds) 0.37 -> 0.38, 73..102 1.3M (4.2) 0.52 -> 0.48; 65..512
+  // bases 750K 1.49 -> 1.57, 137..396 1.3M 2.63 -> 2.70, 193..503 1.3M 4.10 -> 3.53, 200..400
+  // 500K 1.35 -> 1.26, 100..1,000 bases 110K (2.9 rounds) 0.93 -> 0.89; 1,000..10,000 bases
+  // 15K (3.2 rounds) 10.9 -> 12.0, 25K 16.9 -> 12.2, 553..2,544 36K (3.8) 2.79 -> 1.85,
+  // 203..1,831 60K (3.2) 2.13 -> 1.37, 3,000..6,000 bases 15K 9.3 -> 7.3.
+  if (hi <= 256) return tiles >= 4 * round;
+  if (hi <= 768 && !close && len.lo < 160) return false;
+  if (hi > 8192 && len.hi > 4 * len.lo) return tiles >= 4 * round;
   return 4 * tiles >= 11 * round;
 }
-
-// Fewer than two candidates per read (0 reads: unknown).
-static bool few_candidates(uint64_t n, uint64_t reads) { return reads > 0 && n < 2 * reads; }
 
 // lane_words > 0 asks for latency-oriented shapes: a query of more than
 // lane_words words is spread over ceil(words / W) lanes of W <= lane_words

@@ -147,8 +147,27 @@ def test_lanes_of_few_words_without_a_range(plan, entries, faster):
     assert all(W <= 5 for v, L, W in p["shapes"] if 32 * L * W in range(400, 1024)) == faster
 
 
+# path, lengths, candidates, reads and whether bit-sliced shapes are faster: beside the lines between both
+LINES = [(PLAIN, 565, 565, 28_700, 5737, True), (PLAIN, 565, 565, 31_000, 6200, False), (PLAIN, 600, 600, 37_000, 7400, False),
+         (BATCHED, 73, 102, 1_270_000, 115_000, True), (BATCHED, 73, 102, 800_000, 70_000, False),
+         (BATCHED, 193, 503, 1_260_000, 115_000, True), (BATCHED, 137, 396, 1_270_000, 317_000, False),
+         (BATCHED, 217, 503, 656_000, 656_000, False), (BATCHED, 217, 503, 656_000, 150_000, True),
+         (BATCHED, 553, 2544, 35_609, 3200, True), (BATCHED, 203, 1831, 60_330, 5500, True), (BATCHED, 332, 2385, 31_338, 6300, True)]
+
+
+@pytest.mark.parametrize("path,lo,hi,n,reads,faster", LINES)
+def test_bit_sliced_beside_the_lines(plan, path, lo, hi, n, reads, faster):
+    entries = reads * (((lo + hi) // 2 + 127) // 128)
+    assert (plan(path, lo, hi, n, reads, entries=entries)["plan"]["sliced"] > 0) == faster
+
+
 @pytest.mark.parametrize("lo,hi,n,faster", [(613, 916, 5176, True), (114, 824, 9583, True), (100, 1000, 9000, True),
                                             (410, 698, 8447, False), (216, 658, 8746, False)])
 def test_lanes_of_few_words_for_mixed_lengths(plan, lo, hi, n, faster):
     p = plan(BATCHED, lo, hi, n)["plan"]
     assert all(W <= 5 for v, L, W in p["shapes"]) == faster
+
+
+def test_bit_sliced_second_pass(plan):
+    """The cut-off's second pass: mostly one candidate per read."""
+    assert plan(PLAIN, 666, 666, 292_402, 26_582, 0.04, entries=6 * 26_582)["second"]["sliced"] == 1
