@@ -467,7 +467,10 @@ __device__ __forceinline__ void run_words(const DevInputs& in, const Tile& t, co
 
 // Apart from the kernel in the chain class, whose column loops need every register:
 // with the word-parallel tile in line, the loops of single row counts ran up to 13%
-// slower (4,864 bases 4.62 -> 5.31 ms), apart 29 lengths take 0.4% less in all.
+// slower (4,864 bases 4.62 -> 5.31 ms). Which row counts gain changes with whatever the
+// kernel holds: against a kernel with loops for 8..16 rows and the tile in line, 130
+// lengths take from 6% less (32 rows) to 6% more (19 rows), one 14%, 0.2% more in all;
+// with the loops for 17 rows and more and the tile in line 1.2% more in all.
 template <class K>
 __device__ __noinline__ void run_words_apart(const DevInputs& in, const Tile& t, const WarpMem& w, uint32_t m_max,
                                              int lane) {
