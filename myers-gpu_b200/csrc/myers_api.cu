@@ -488,6 +488,10 @@ static bool sliced_batch(const Batch& b, bool batched, uint32_t& spread) {
   // Nor with a read or more of its own per candidate, which short tiles don't hide:
   // 104..331 bases 1.1M of one read each 1.65 -> 2.51, 217..503 bases 660K 2.37 -> 3.08.
   if (hi <= 768 && few_candidates(n, b.reads)) return false;
+  // The cut-off's prefixes are multiples of 32 rows, so few shapes, which large
+  // batches fill: reads of 100..1,000 bases at 0.2 m (64..480 rows) 320K (4.2 rounds) 1.00
+  // -> 1.02, 969K (12.8) 4.57 -> 3.83; at 0.08 m (32..192 rows) 22M (72) 53.2 -> 45.0.
+  if (b.prefixes && tiles >= 8 * round) return true;
   if (len.lo < kSlicedMinRows || len.hi > kSlicedMaxRows) return len.hi > 512 && tiles >= 5 * round;
   // 70..150 bases 660K (2.2 rounds) 0.37 -> 0.38, 73..102 1.3M (4.2) 0.52 -> 0.48; 65..512
   // bases 750K 1.49 -> 1.57, 137..396 1.3M 2.63 -> 2.70, 193..503 1.3M 4.10 -> 3.53, 200..400
@@ -875,7 +879,9 @@ int myers::cutoff_plans(PlanTable& plan, PlanTable& plan2, const uint8_t* presen
     b.lengths = m1;
     b.bucketed = bucketed;
     b.by_words = by_words;
+    b.prefixes = true;
     const int st = build_plan(plan, w1, batched, 0, b);
+    b.prefixes = false;
     b.reads = n;
     b.mean = mean;
     b.lengths = m2;

@@ -319,6 +319,7 @@ struct Batch {
   uint32_t mean = 0;      // bases of a read on average (0: unknown)
   uint64_t sliced_n = 0;  // candidates expected, where they are not n (the cut-off's second pass)
   bool bucketed = false;  // the candidates will be classified in any case: name every shape of the word counts present
+  bool prefixes = false;  // the lengths are those of the cut-off's prefixes
   bool by_words = false;  // admit queries by their word counts alone
   bool unshared = true;   // no other batches share the device (a server's do)
 };

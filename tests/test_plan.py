@@ -171,3 +171,9 @@ def test_lanes_of_few_words_for_mixed_lengths(plan, lo, hi, n, faster):
 def test_bit_sliced_second_pass(plan):
     """The cut-off's second pass: mostly one candidate per read."""
     assert plan(PLAIN, 666, 666, 292_402, 26_582, 0.04, entries=6 * 26_582)["second"]["sliced"] == 1
+
+
+@pytest.mark.parametrize("cut,n,faster", [(0.08, 22_000_000, True), (0.2, 969_000, True), (0.2, 320_000, False)])
+def test_bit_sliced_first_pass(plan, cut, n, faster):
+    """The cut-off's first pass on the batched path: prefixes of a few row counts."""
+    assert (plan(BATCHED, 100, 1000, n, n // 11, cut, entries=4 * (n // 11))["first"]["sliced"] > 0) == faster
